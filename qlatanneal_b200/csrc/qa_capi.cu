@@ -23,6 +23,7 @@
 #include "qa_pm1.cuh"
 #include "qa_pt.cuh"
 #include "qa_ingest.cuh"
+#include "qa_dense.cuh"
 
 using namespace qa;
 
@@ -204,6 +205,7 @@ struct qa_problem {
     int tc_int8 = -1;  // -1 unknown, 0 no, 1 yes
     int8_t *J8 = nullptr;
     int tc_ldj = 0;
+    bool plain_j = false;  // dense: every coupling finite and below 2^126
     double c = 0.0;
     std::vector<void *> allocs;
     ProbDev dev{};
@@ -284,6 +286,7 @@ int finish_problem(qa_problem *P) {
     P->dev.T = P->T;
     P->dev.m = P->m;
     P->dev.c = P->c;
+    P->dev.ldj = dense_ld(P->n);
     HostStage &st = P->ctx->stage;
     if (P->fix.empty()) st.clear();  // nothing staged for this problem
     std::vector<size_t> roff;
@@ -511,7 +514,7 @@ int tc_prepare(qa_ctx *ctx, qa_problem *P) {
     QA_CK(cudaMallocAsync(reinterpret_cast<void **>(&d_ok), sizeof(int), ctx->stream));
     const int one = 1;
     QA_CK(cudaMemcpyAsync(d_ok, &one, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    tc_int8_check_kernel<<<256, 256, 0, ctx->stream>>>(P->dev.J32, (long long)n * n, d_ok);
+    tc_int8_check_kernel<<<256, 256, 0, ctx->stream>>>(P->dev.J32, (long long)n * P->dev.ldj, d_ok);
     QA_CK(cudaGetLastError());
     int ok = 0;
     QA_CK(cudaMemcpyAsync(&ok, d_ok, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
@@ -524,7 +527,7 @@ int tc_prepare(qa_ctx *ctx, qa_problem *P) {
     P->allocs.push_back(d);
     P->J8 = static_cast<int8_t *>(d);
     P->tc_ldj = ldj;
-    tc_pack_couplings_kernel<<<256, 256, 0, ctx->stream>>>(P->dev.J32, n, ldj, rows, P->J8);
+    tc_pack_couplings_kernel<<<256, 256, 0, ctx->stream>>>(P->dev.J32, n, P->dev.ldj, ldj, rows, P->J8);
     QA_CK(cudaGetLastError());
     P->tc_int8 = 1;
     return QA_OK;
@@ -610,6 +613,7 @@ int exact_energies(qa_ctx *ctx, int kind, const ProbDev *d_probs, const Layout &
 struct RingPlan {
     bool pm1 = false;     // ring_pm1_kernel
     bool sparse = false;  // ring_sparse_kernel
+    bool dense = false;   // ring_dense_kernel
     bool own_fields() const { return pm1 || sparse; }  // no field cache to initialise
     int gbytes = 4;       // pm1: bytes per field (4 int32, 2 int16)
     bool jw_smem = true;  // pm1: J bits in shared memory
@@ -626,7 +630,7 @@ struct RingPlan {
 // fields, int16 fields with J read from L2.  P <= 64 (worldlines are 64-bit
 // columns) and n <= 2048.  Anything else runs ring_kernel.
 int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, int P, int n_max, RingPlan *pl,
-               bool clusters = false, bool ref_order = false) {
+               int n_rings, bool clusters = false, bool ref_order = false) {
     pl->W = std::max(1, std::min(32, (P + 1) / 2));
     if (ctx->tune.warps_per_ring > 0) pl->W = std::max(1, std::min({32, P, ctx->tune.warps_per_ring}));
     pl->ref_order = ref_order;
@@ -683,6 +687,21 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
         pl->smem_fields = 0;
         return QA_OK;
     }
+    // dense couplings of any value: ring_dense_kernel
+    pl->dense = !clusters && kind == K_DENSE && P <= 64 && !std::getenv("QA_DISABLE_DENSE") &&
+                dense_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin;
+    for (int p = 0; p < np && pl->dense; ++p) pl->dense = probs[p]->plain_j;
+    if (pl->dense) {
+        pl->smem = dense_smem_bytes(P, n_max, ref_order);
+        // one warp per slice up to 16 (the kernel's 128 registers a thread);
+        // 8 where the rings are at least two waves and blocks are few (n <= 256):
+        // two rings on an SM then beat one with twice the warps (P = 32,
+        // 600 rings: n = 24 23.3 -> 17.7 ms, n = 64 36.8 -> 28.3, n = 200
+        // 69.9 -> 66.4; 300 rings of n = 900 25.1 -> 28.2, so not there)
+        if (ctx->tune.warps_per_ring <= 0) pl->W = std::min(P, n_rings >= 2 * ctx->sms && n_max <= 256 ? 8 : 16);
+        pl->W = std::min(pl->W, 16);
+        return QA_OK;
+    }
     // generic kernel in qanneal's order: one warp per slice for P <= 16, as
     // for the +-1 kernel (HUBO n=1024 P=16: 11.5% faster)
     if (ref_order && ctx->tune.warps_per_ring <= 0 && P <= 16) pl->W = P;
@@ -704,6 +723,10 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
     if (!placed) pl->smem = ring_smem_bytes(P, n_max, pl->W, false, ref_order, false);
     if (pl->smem > (size_t)ctx->smem_optin) return fail(QA_ERR_ARG, "ring state does not fit in shared memory.");
     return QA_OK;
+}
+
+static void (*dense_kernel(const RingPlan &pl))(RingParams) {
+    return pl.ref_order ? ring_dense_kernel<true> : ring_dense_kernel<false>;
 }
 
 // One launch of the planned ring kernel over steps [rp.step0, rp.step1).
@@ -824,6 +847,13 @@ int launch_rings(qa_ctx *ctx, int kind, const RingPlan &pl, RingParams rp, int n
         QA_CK(cudaGetLastError());
         return QA_OK;
     }
+    if (pl.dense) {
+        auto kern = dense_kernel(pl);
+        QA_TRY(opt_in_smem(ctx, (const void *)kern, pl.smem));
+        kern<<<n_rings, 32 * pl.W, pl.smem, strm>>>(rp);
+        QA_CK(cudaGetLastError());
+        return QA_OK;
+    }
     if (pl.sparse) {
         QA_TRY(opt_in_smem(ctx, (const void *)ring_sparse_kernel, pl.smem));
         ring_sparse_kernel<<<n_rings, 32 * pl.W, pl.smem, strm>>>(rp);
@@ -894,6 +924,8 @@ static bool rotation_pays(qa_ctx *ctx, int kind, const RingPlan &pl, int nr) {
                                             : (const void *)ring_pm1_kernel<short, false>);
     else if (pl.sparse)
         kern = (const void *)ring_sparse_kernel;
+    else if (pl.dense)
+        kern = (const void *)dense_kernel(pl);
     else
         dispatch_kind(kind, [&](auto Kd) { kern = (const void *)ring_kernel<decltype(Kd)::value>; });
     if (opt_in_smem(ctx, kern, pl.smem) != QA_OK) return false;
@@ -947,8 +979,9 @@ static int plan_models(qa_ctx *ctx, const qa_problem *const *probs, int np, int 
     std::vector<ModelRun> mr(np);
     bool pays = false;
     for (int m = 0; m < np; ++m) {
-        QA_TRY(plan_rings(ctx, probs + m, 1, kind, P, probs[m]->n, &mr[m].pl, clusters, ref_order));
-        if (mr[m].pl.pm1 != set_pl.pm1 || mr[m].pl.sparse != set_pl.sparse) mr[m].pl = set_pl;
+        QA_TRY(plan_rings(ctx, probs + m, 1, kind, P, probs[m]->n, &mr[m].pl, nr, clusters, ref_order));
+        if (mr[m].pl.pm1 != set_pl.pm1 || mr[m].pl.sparse != set_pl.sparse || mr[m].pl.dense != set_pl.dense)
+            mr[m].pl = set_pl;
         mr[m].g0 = m * (nr / np);
         mr[m].nr = nr / np;
         pays = pays || 5 * mr[m].pl.smem <= 4 * set_pl.smem;
@@ -1232,12 +1265,13 @@ static int derive_dense(qa_problem *P) {
     QA_CK(cudaMemsetAsync(d_flag, 0, sizeof(int), ctx->stream));
     QA_CK(cudaMemsetAsync(const_cast<uint32_t *>(P->dev.Jw), 0, sizeof(uint32_t) * (size_t)nw * np, ctx->stream));
     dense_derive_kernel<<<dim3(nw, nw), dim3(kIngestTile, 8), 0, ctx->stream>>>(
-        P->dev.J64, n, const_cast<float *>(P->dev.J32), const_cast<uint32_t *>(P->dev.Jw), np, d_flag);
+        P->dev.J64, n, P->dev.ldj, const_cast<float *>(P->dev.J32), const_cast<uint32_t *>(P->dev.Jw), np, d_flag);
     QA_CK(cudaGetLastError());
-    int not_pm1 = 0;
-    QA_CK(cudaMemcpyAsync(&not_pm1, d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
+    int flags = 0;
+    QA_CK(cudaMemcpyAsync(&flags, d_flag, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
     QA_CK(cudaStreamSynchronize(ctx->stream));
-    if (not_pm1) P->dev.Jw = nullptr;
+    if (flags & 1) P->dev.Jw = nullptr;
+    P->plain_j = !(flags & 2);
     return QA_OK;
 }
 
@@ -1258,7 +1292,7 @@ int qa_problem_dense(qa_ctx *ctx, int n, const double *h, const double *J, doubl
     int rc = common_h(P, h);
     if (rc == QA_OK) rc = upload(P, J, (size_t)n * n, &P->dev.J64);
     if (rc == QA_OK) {
-        reserve_array(P, (size_t)n * n, &P->dev.J32);
+        reserve_array(P, (size_t)n * dense_ld(n), &P->dev.J32);
         reserve_array(P, (size_t)P->nw * pm1_npad(n), &P->dev.Jw);
         rc = finish_problem(P);
     }
@@ -1285,7 +1319,7 @@ int qa_problem_qubo(qa_ctx *ctx, int n, const double *Q, double *h_out, double *
     reserve_array(P, (size_t)n, &P->dev.h32);
     reserve_array(P, (size_t)n, &P->dev.h64);
     reserve_array(P, (size_t)n * n, &P->dev.J64);
-    reserve_array(P, (size_t)n * n, &P->dev.J32);
+    reserve_array(P, (size_t)n * dense_ld(n), &P->dev.J32);
     reserve_array(P, (size_t)P->nw * pm1_npad(n), &P->dev.Jw);
     int rc = finish_problem(P);
     double *d_Q = nullptr;
@@ -1929,7 +1963,7 @@ static int sqa_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_proble
 
     QA_CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     RingPlan pl;
-    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, prm->cluster_sweeps > 0 || traces,
+    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, nr, prm->cluster_sweeps > 0 || traces,
                       ctx->update_order == QA_ORDER_REFERENCE));
     // dense +-1 couplings: the bit-packed kernel builds its fields in-kernel
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, P, n_max, L.nw_max, DOM_INIT, !pl.own_fields(),
@@ -2271,7 +2305,7 @@ int qa_sqa_opt_run(qa_ctx *ctx, const qa_problem *const *problems, int n_problem
 
     QA_CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     RingPlan pl;
-    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, cls > 0, ctx->update_order == QA_ORDER_REFERENCE));
+    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, nr, cls > 0, ctx->update_order == QA_ORDER_REFERENCE));
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, P, n_max, L.nw_max, DOM_INIT,
                       !pl.own_fields(), problems, n_problems, &L, d_cnt + 4));
     RingParams rp{};
@@ -2684,7 +2718,7 @@ static int sqapt_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_prob
     }
     RingPlan pl;
     // classical parallel tempering keeps its ascending order (parallel_tempering.cpp:36-122)
-    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, prm->cluster_sweeps > 0,
+    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, nr, prm->cluster_sweeps > 0,
                       !classical && ctx->update_order == QA_ORDER_REFERENCE));
     QA_CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, P, n_max, L.nw_max, DOM_INIT, !pl.own_fields(),
@@ -2901,7 +2935,7 @@ int qa_sqapt_opt_run(qa_ctx *ctx, const qa_problem *const *problems, int n_probl
         QA_CK(cudaStreamSynchronize(ctx->stream));
     }
     RingPlan pl;
-    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, cls > 0, ctx->update_order == QA_ORDER_REFERENCE));
+    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, nr, cls > 0, ctx->update_order == QA_ORDER_REFERENCE));
     QA_CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, P, n_max, L.nw_max, DOM_INIT,
                       !pl.own_fields(), problems, n_problems, &L, d_cnt + 4));
@@ -3295,7 +3329,7 @@ static int chi_stage1(qa_ctx *ctx, const qa_problem *const *problems, int n_prob
     h2d += (int64_t)(sizeof(ProbDev) * n_problems + sizeof(RingDev) * nr + 2 * sizeof(float) * Pts +
                      sizeof(int) * nof.size() + sizeof(double) * nr);
     RingPlan pl;
-    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl));
+    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, nr));
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, P, n_max, L.nw_max, DOM_PILOT_INIT,
                       !pl.own_fields(), problems, n_problems, &L, d_cnt + 4));
     RingParams rp{};
@@ -3485,7 +3519,7 @@ int qa_chi_run(qa_ctx *ctx, const qa_problem *const *problems, int n_problems, c
                          (sizeof(double) + sizeof(int)) * nr);
     }
     RingPlan pl;
-    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl));
+    QA_TRY(plan_rings(ctx, problems, n_problems, kind, P, n_max, &pl, nr));
     QA_CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, P, n_max, L.nw_max, DOM_PROD_INIT, !pl.own_fields(),
                       problems, n_problems, &L, d_cnt + 4));

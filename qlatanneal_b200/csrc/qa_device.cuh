@@ -133,7 +133,9 @@ struct ProbDev {
     double c;
     const float *h32;
     const double *h64;
-    // dense: J32 row-major n x n (symmetric, zero diagonal), J64 as given
+    // dense: J32 row-major n x n (symmetric, zero diagonal), rows ldj apart
+    // (padding 0), J64 as given
+    int ldj;
     const float *J32;
     const double *J64;
     // sparse: merged adjacency CSR + original edge list (float64 energy)
@@ -178,7 +180,7 @@ template <int KIND>
 __device__ __forceinline__ void apply_flip(const ProbDev &P, float *g, const uint32_t *S, int j, int so, int lane) {
     const float cf = so > 0 ? -2.0f : 2.0f;
     if (KIND == K_DENSE) {
-        const float *row = P.J32 + (size_t)j * P.n;
+        const float *row = P.J32 + (size_t)j * P.ldj;
         for (int m = lane; m < P.n; m += 32)
             if (m != j) g[m] = __fadd_rn(g[m], __fmul_rn(cf, __ldg(row + m)));
     } else if (KIND == K_SPARSE) {
@@ -242,7 +244,7 @@ __device__ __forceinline__ double field_exact64(const ProbDev &P, const uint32_t
     if (KIND == K_DENSE) {
         // J32 is symmetric: read column i (coalesced across the lanes' rows)
         for (int j = 0; j < P.n; ++j) {
-            const double w = (double)__ldg(P.J32 + (size_t)j * P.n + i);
+            const double w = (double)__ldg(P.J32 + (size_t)j * P.ldj + i);
             acc = __dadd_rn(acc, spin_of(S, j) > 0 ? w : -w);
         }
     } else if (KIND == K_SPARSE) {

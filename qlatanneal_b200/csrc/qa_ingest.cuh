@@ -56,12 +56,14 @@ __global__ void qubo_rows_kernel(const double *__restrict__ Q, int n, double *__
 // Derived dense arrays, one CTA (32 x 8 threads) per 32 x 32 tile (row tile
 // blockIdx.y, column tile blockIdx.x).  The upper triangle of J64 defines the
 // model (DenseIsing::energy reads i < j):
-//   J32[i][j] = (float) J64[min(i,j)][max(i,j)] for i != j, 0 on the diagonal
+//   J32[i][j] = (float) J64[min(i,j)][max(i,j)] for i != j, 0 on the diagonal,
+//   rows ld >= n apart with zeros behind them
 //   Jw[q * np + m]: bit (j & 31) of row m, column word q = (J32[m][j] > 0), j != m
-//   *not_pm1 = 1 when an upper off-diagonal entry is neither +1 nor -1.
+//   *flags: bit 0 when an upper off-diagonal entry is neither +1 nor -1, bit 1
+//   when one is 2^126 or more in magnitude or not finite.
 // Jw must be zeroed beforehand (rows n .. np-1 stay 0).
-__global__ void dense_derive_kernel(const double *__restrict__ J64, int n, float *__restrict__ J32,
-                                    uint32_t *__restrict__ Jw, int np, int *__restrict__ not_pm1) {
+__global__ void dense_derive_kernel(const double *__restrict__ J64, int n, int ld, float *__restrict__ J32,
+                                    uint32_t *__restrict__ Jw, int np, int *__restrict__ flags) {
     __shared__ double S[kIngestTile][kIngestTile + 1];  // J64[a0 + y][b0 + x]
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int bx = blockIdx.x, by = blockIdx.y;
@@ -72,19 +74,21 @@ __global__ void dense_derive_kernel(const double *__restrict__ J64, int n, float
     }
     __syncthreads();
     const int r0 = kIngestTile * by, c0 = kIngestTile * bx;
-    bool bad = false;
+    bool bad = false, huge = false;
     for (int y = ty; y < kIngestTile; y += blockDim.y) {
         const int i = r0 + y, j = c0 + tx;
         const bool in = i < n && j < n;
         const int lo = min(i, j), hi = max(i, j);
         const double v = (in && i != j) ? S[lo - a0][hi - b0] : 0.0;
         if (in && i < j && v != 1.0 && v != -1.0) bad = true;
-        if (in) J32[(size_t)i * n + j] = i == j ? 0.0f : __double2float_rn(v);
         const float f = __double2float_rn(v);
+        if (!(fabsf(f) < 8.507059e37f)) huge = true;  // 2^126
+        if (i < n && j < ld) J32[(size_t)i * ld + j] = f;  // v is 0 on the diagonal and behind the row
         const uint32_t word = __ballot_sync(0xffffffffu, in && i != j && f > 0.0f);
         if (tx == 0 && i < n) Jw[(size_t)bx * np + i] = word;
     }
-    if (__any_sync(0xffffffffu, bad) && tx == 0) *not_pm1 = 1;
+    const int fl = (__any_sync(0xffffffffu, bad) ? 1 : 0) | (__any_sync(0xffffffffu, huge) ? 2 : 0);
+    if (fl && tx == 0) atomicOr(flags, fl);
 }
 
 }  // namespace qa

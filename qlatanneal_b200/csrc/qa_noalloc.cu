@@ -155,6 +155,7 @@ extern "C" int qa_sa_dense_run_noalloc(int device, void *stream, int n, const do
     pd.h32 = reinterpret_cast<const float *>(base + o_h32);
     pd.h64 = d_h;
     pd.J32 = reinterpret_cast<const float *>(base + o_J32);
+    pd.ldj = n;
     pd.J64 = d_J;
     std::vector<RingDev> rings(reads);
     for (int r = 0; r < reads; ++r) {

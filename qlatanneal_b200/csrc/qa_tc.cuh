@@ -192,12 +192,12 @@ __global__ void __launch_bounds__(128, 1) tc_fields_kernel(TcFieldParams p) {
 
 // The int8 coupling rows of a dense problem with integer couplings in
 // [-127, 127]: [rows][ldj], zero padded, zero diagonal (J32 has one).
-__global__ void tc_pack_couplings_kernel(const float *J32, int n, int ldj, int rows, int8_t *J8) {
+__global__ void tc_pack_couplings_kernel(const float *J32, int n, int ld32, int ldj, int rows, int8_t *J8) {
     const long long total = (long long)rows * ldj;
     for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
          idx += (long long)gridDim.x * blockDim.x) {
         const int m = (int)(idx / ldj), j = (int)(idx - (long long)m * ldj);
-        J8[idx] = (m < n && j < n) ? (int8_t)(int)J32[(long long)m * n + j] : (int8_t)0;
+        J8[idx] = (m < n && j < n) ? (int8_t)(int)J32[(long long)m * ld32 + j] : (int8_t)0;
     }
 }
 
