@@ -225,7 +225,7 @@ namespace {
 enum WsSlot { W_PROBS, W_RINGS, W_SPINS, W_FIELDS, W_A, W_T4, W_SUM, W_BESTE, W_BESTSTEP, W_BITS, W_CNT, W_EXACT,
               W_PROBOF, W_MIN, W_BOND, W_MAG, W_SLOT, W_RIN, W_BSLOT, W_FBITS, W_AVG, W_SWP, W_BPJP, W_JP,
               W_BSAMP, W_SSAVE, W_FSAVE, W_CBESTE, W_CBSTEP, W_CBITS, W_CBOND, W_FLAG, W_QSTAGE,
-              W_TRB, W_TRE, W_TREB, W_TREE, W_RSPIN, W_DRIFT, W_ORDER, W_OSCR, W_COUNT };
+              W_TRB, W_TRE, W_TREB, W_TREE, W_RSPIN, W_DRIFT, W_ORDER, W_OSCR, W_ROWSUM, W_COUNT };
 static_assert(W_COUNT <= qa_ctx::kWsSlots, "qa_ctx::ws has a slot per WsSlot");
 
 int ws_get(qa_ctx *ctx, int slot, size_t bytes, void **out) {
@@ -600,6 +600,26 @@ int exact_energies(qa_ctx *ctx, int kind, const ProbDev *d_probs, const Layout &
     QA_TRY(ws_get(ctx, W_PROBOF, sizeof(int) * prob_of.size(), &v));
     int *d_pof = static_cast<int *>(v);
     QA_CK(cudaMemcpyAsync(d_pof, prob_of.data(), sizeof(int) * prob_of.size(), cudaMemcpyHostToDevice, ctx->stream));
+    // from n = 65 on two kernels over row tiles (1 state at n = 24: 8.0 us in one
+    // kernel, 10.9 in two; n = 64: 16.0 / 15.2; 32 states at n = 96: 26.4 / 19.6)
+    if (kind == K_DENSE && L.nw_max > 2) {
+        // the row sums of at most 64 MB of states at a time
+        const int count = (int)L.rings.size(), n_max = 32 * L.nw_max, per = 8 * kExactPer;
+        const size_t fit = std::min<size_t>(((size_t)64 << 20) / (8 * (size_t)n_max), (size_t)65535 * per);
+        const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)count, fit));
+        double *d_rs;
+        QA_TRY(ws_get(ctx, W_ROWSUM, sizeof(double) * (size_t)chunk * n_max, &v));
+        d_rs = static_cast<double *>(v);
+        for (int s0 = 0; s0 < count; s0 += chunk) {
+            const int c = std::min(chunk, count - s0);
+            const uint32_t *b = d_bits + (size_t)s0 * L.nw_max;
+            dense_row_sums_kernel<<<dim3((n_max + 31) / 32, (c + per - 1) / per), 256, 0, ctx->stream>>>(
+                d_probs, d_pof + s0, b, L.nw_max, c, n_max, d_rs);
+            dense_exact_kernel<<<c, 32, 0, ctx->stream>>>(d_probs, d_pof + s0, b, L.nw_max, n_max, d_rs, d_exact + s0);
+        }
+        QA_CK(cudaGetLastError());
+        return QA_OK;
+    }
     int rc = QA_OK;
     dispatch_kind(kind, [&](auto K) {
         exact_energy_kernel<decltype(K)::value><<<(unsigned)L.rings.size(), 32, L.nw_max * 4, ctx->stream>>>(
