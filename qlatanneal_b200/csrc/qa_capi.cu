@@ -206,6 +206,7 @@ struct qa_problem {
     int8_t *J8 = nullptr;
     int tc_ldj = 0;
     bool plain_j = false;  // dense: every coupling finite and below 2^126
+    bool int8_j = false;   // dense: every coupling an integer in [-127, 127]
     double c = 0.0;
     std::vector<void *> allocs;
     ProbDev dev{};
@@ -508,19 +509,8 @@ int upload_common(qa_ctx *ctx, const qa_problem *const *probs, int np, const Lay
 int tc_prepare(qa_ctx *ctx, qa_problem *P) {
     if (P->tc_int8 >= 0) return QA_OK;
     P->tc_int8 = 0;
-    if (P->kind != K_DENSE || !P->dev.J32) return QA_OK;
+    if (P->kind != K_DENSE || !P->dev.J32 || !P->int8_j) return QA_OK;
     const int n = P->n;
-    int *d_ok = nullptr;
-    QA_CK(cudaMallocAsync(reinterpret_cast<void **>(&d_ok), sizeof(int), ctx->stream));
-    const int one = 1;
-    QA_CK(cudaMemcpyAsync(d_ok, &one, sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    tc_int8_check_kernel<<<256, 256, 0, ctx->stream>>>(P->dev.J32, (long long)n * P->dev.ldj, d_ok);
-    QA_CK(cudaGetLastError());
-    int ok = 0;
-    QA_CK(cudaMemcpyAsync(&ok, d_ok, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
-    QA_CK(cudaStreamSynchronize(ctx->stream));
-    QA_CK(cudaFreeAsync(d_ok, ctx->stream));
-    if (!ok) return QA_OK;
     const int ldj = (n + TC_K - 1) / TC_K * TC_K, rows = (n + TC_N - 1) / TC_N * TC_N;
     void *d = nullptr;
     QA_CK(cudaMalloc(&d, (size_t)rows * ldj));
@@ -1292,6 +1282,7 @@ static int derive_dense(qa_problem *P) {
     QA_CK(cudaStreamSynchronize(ctx->stream));
     if (flags & 1) P->dev.Jw = nullptr;
     P->plain_j = !(flags & 2);
+    P->int8_j = !(flags & 4);
     return QA_OK;
 }
 

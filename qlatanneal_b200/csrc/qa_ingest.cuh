@@ -60,7 +60,8 @@ __global__ void qubo_rows_kernel(const double *__restrict__ Q, int n, double *__
 //   rows ld >= n apart with zeros behind them
 //   Jw[q * np + m]: bit (j & 31) of row m, column word q = (J32[m][j] > 0), j != m
 //   *flags: bit 0 when an upper off-diagonal entry is neither +1 nor -1, bit 1
-//   when one is 2^126 or more in magnitude or not finite.
+//   when one is 2^126 or more in magnitude or not finite, bit 2 when one is no
+//   integer in [-127, 127].
 // Jw must be zeroed beforehand (rows n .. np-1 stay 0).
 __global__ void dense_derive_kernel(const double *__restrict__ J64, int n, int ld, float *__restrict__ J32,
                                     uint32_t *__restrict__ Jw, int np, int *__restrict__ flags) {
@@ -74,7 +75,7 @@ __global__ void dense_derive_kernel(const double *__restrict__ J64, int n, int l
     }
     __syncthreads();
     const int r0 = kIngestTile * by, c0 = kIngestTile * bx;
-    bool bad = false, huge = false;
+    bool bad = false, huge = false, wide = false;
     for (int y = ty; y < kIngestTile; y += blockDim.y) {
         const int i = r0 + y, j = c0 + tx;
         const bool in = i < n && j < n;
@@ -83,11 +84,13 @@ __global__ void dense_derive_kernel(const double *__restrict__ J64, int n, int l
         if (in && i < j && v != 1.0 && v != -1.0) bad = true;
         const float f = __double2float_rn(v);
         if (!(fabsf(f) < 8.507059e37f)) huge = true;  // 2^126
+        if (!(f == rintf(f) && fabsf(f) <= 127.0f)) wide = true;
         if (i < n && j < ld) J32[(size_t)i * ld + j] = f;  // v is 0 on the diagonal and behind the row
         const uint32_t word = __ballot_sync(0xffffffffu, in && i != j && f > 0.0f);
         if (tx == 0 && i < n) Jw[(size_t)bx * np + i] = word;
     }
-    const int fl = (__any_sync(0xffffffffu, bad) ? 1 : 0) | (__any_sync(0xffffffffu, huge) ? 2 : 0);
+    const int fl = (__any_sync(0xffffffffu, bad) ? 1 : 0) | (__any_sync(0xffffffffu, huge) ? 2 : 0) |
+                   (__any_sync(0xffffffffu, wide) ? 4 : 0);
     if (fl && tx == 0) atomicOr(flags, fl);
 }
 

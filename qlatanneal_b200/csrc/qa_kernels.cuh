@@ -132,6 +132,11 @@ __global__ void init_fields_kernel(const ProbDev *probs, const RingDev *rings, c
         g[i] = field_init_one<KIND>(Pd, sS, i);
 }
 
+// v or -v, by bit b of w (1: -v): two integer operations on the high word.
+__device__ __forceinline__ double neg_by_bit(double v, uint32_t w, int b) {
+    return __hiloint2double(__double2hiint(v) ^ (int)((w << (31 - b)) & 0x80000000u), __double2loint(v));
+}
+
 // Drift of the float32 field caches: the largest |g - float64 recompute from
 // the same float32 couplings| over every (ring, slice, spin) of the grid
 // (blockIdx.x ring, blockIdx.y slice).  Non-negative doubles order as their
@@ -872,7 +877,7 @@ __global__ void exact_energy_kernel(const ProbDev *probs, const int *prob_of, co
 // here a CTA of 8 warps takes 32 rows of 8 * kExactPer states: the couplings come
 // through shared memory in 32 x 32 tiles (coalesced, read once for all the
 // states), each lane sums one row of kExactPer states.  Both kernels, 128 states
-// at n = 2000: 8314 -> 209 us; 128 at n = 1000: 2106 -> 107 us.
+// at n = 2000: 8314 -> 181 us; 128 at n = 1000: 2106 -> 93 us.
 //   rs[state][i] = s_i sum_{j > i} J_ij s_j    (row order)
 constexpr int kExactPer = 2;
 static __global__ void __launch_bounds__(256) dense_row_sums_kernel(const ProbDev *probs, const int *prob_of,
@@ -907,12 +912,11 @@ static __global__ void __launch_bounds__(256) dense_row_sums_kernel(const ProbDe
                 uint32_t w[kExactPer];
 #pragma unroll
                 for (int k = 0; k < kExactPer; ++k) w[k] = ~__ldg(sw[k] + (c0 >> 5));
-#pragma unroll 8
+#pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     const double v = tile[lane][j];
 #pragma unroll
-                    for (int k = 0; k < kExactPer; ++k)
-                        acc[k] = __dadd_rn(acc[k], ((w[k] >> j) & 1u) ? -v : v);
+                    for (int k = 0; k < kExactPer; ++k) acc[k] = __dadd_rn(acc[k], neg_by_bit(v, w[k], j));
                 }
             }
 #pragma unroll

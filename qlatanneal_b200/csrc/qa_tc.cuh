@@ -201,13 +201,4 @@ __global__ void tc_pack_couplings_kernel(const float *J32, int n, int ld32, int 
     }
 }
 
-// 1 when every coupling is an integer in [-127, 127].
-__global__ void tc_int8_check_kernel(const float *J32, long long count, int *ok) {
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < count;
-         i += (long long)gridDim.x * blockDim.x) {
-        const float v = J32[i];
-        if (!(v == rintf(v) && fabsf(v) <= 127.0f)) atomicExch(ok, 0);
-    }
-}
-
 }  // namespace qa

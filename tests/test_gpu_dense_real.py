@@ -97,3 +97,18 @@ def test_huge_couplings_keep_the_generic_kernel(monkeypatch):
     a, b = _both(monkeypatch, lambda: qa.SQAAnnealer(model, s, 4).run_reads(1, 1, reads=3, seed=2))
     for x, y in zip(a, b):
         np.testing.assert_array_equal(x.best_state.as_array(), y.best_state.as_array())
+
+
+def test_batch_of_uneven_models_equals_single_runs():
+    """Exact energies (16 states a CTA) where a CTA's states belong to two models."""
+    models = [qa.DenseIsing(*dense_real(n, 20 + n)) for n in (130, 65, 97, 300)]
+    s = qa.SQASchedule.from_vectors([0.5, 2.0, 6.0], [2.0, 1.0, 0.1])
+    both = qa.BatchRunner().sqa(models, s, 3, reads=5, worldline_sweeps=1, seed=4)
+    sa = qa.BatchRunner().anneal(models, qa.AnnealSchedule.from_betas([0.2, 1.0]), 2, reads=5, seed=4)
+    for m, x, y in zip(models, both, sa):
+        for got, want in ((x, qa.SQAAnnealer(m, s, 3).run_reads(1, 1, reads=5, seed=4)),
+                          (y, qa.Annealer(m, qa.AnnealSchedule.from_betas([0.2, 1.0])).run_reads(2, 5, seed=4))):
+            for a, b in zip(got, want):
+                np.testing.assert_array_equal(a.best_state.as_array(), b.best_state.as_array())
+                assert a.best_energy == b.best_energy
+                np.testing.assert_array_equal(a.energy_trace, b.energy_trace)
