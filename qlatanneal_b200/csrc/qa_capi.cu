@@ -24,6 +24,7 @@
 #include "qa_pt.cuh"
 #include "qa_ingest.cuh"
 #include "qa_dense.cuh"
+#include "qa_slab.cuh"
 
 using namespace qa;
 
@@ -624,7 +625,9 @@ struct RingPlan {
     bool pm1 = false;     // ring_pm1_kernel
     bool sparse = false;  // ring_sparse_kernel
     bool dense = false;   // ring_dense_kernel
-    bool own_fields() const { return pm1 || sparse; }  // no field cache to initialise
+    bool slab = false;    // ring_slab_kernel
+    bool wide = false;    // slab: 64-bit worldline words (P > 32)
+    bool own_fields() const { return pm1 || sparse || slab; }  // no field cache to initialise
     int gbytes = 4;       // pm1: bytes per field (4 int32, 2 int16)
     bool jw_smem = true;  // pm1: J bits in shared memory
     bool ref_order = false;  // qanneal's update order (else the parity checkerboard)
@@ -687,6 +690,17 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
             pl->W = P;
         return QA_OK;
     }
+    // sparse rows in neighbour records: spins outside, slices inside
+    pl->slab = !clusters && kind == K_SPARSE && P <= 64 && !std::getenv("QA_DISABLE_SPARSE_INT") &&
+               !std::getenv("QA_DISABLE_SLAB") && slab_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin;
+    for (int p = 0; p < np && pl->slab; ++p) pl->slab = probs[p]->dev.spslab != nullptr;
+    if (pl->slab) {
+        pl->wide = P > 32;
+        pl->smem = slab_smem_bytes(P, n_max, ref_order);
+        pl->smem_fields = 0;
+        pl->W = std::min(8, (n_max + 127) / 128);
+        return QA_OK;
+    }
     // sparse integer couplings: fields on demand, worldline sums from bits
     pl->sparse = !clusters && kind == K_SPARSE && P <= 64 &&
                  sparse_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin &&
@@ -735,6 +749,11 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
     return QA_OK;
 }
 
+static void (*slab_kernel(const RingPlan &pl))(RingParams) {
+    if (pl.wide)
+        return pl.ref_order ? ring_slab_kernel<unsigned long long, true> : ring_slab_kernel<unsigned long long, false>;
+    return pl.ref_order ? ring_slab_kernel<uint32_t, true> : ring_slab_kernel<uint32_t, false>;
+}
 static void (*dense_kernel(const RingPlan &pl))(RingParams) {
     return pl.ref_order ? ring_dense_kernel<true> : ring_dense_kernel<false>;
 }
@@ -774,7 +793,7 @@ static int opt_in_smem(qa_ctx *ctx, const void *kern, size_t smem) {
 constexpr size_t kOrderBudget = (size_t)256 << 20;
 
 static int ord_rows_per_step(const RingPlan &pl, const RingParams &rp) {
-    return rp.spb + (pl.pm1 || pl.sparse ? 0 : rp.cls) + rp.wls;
+    return rp.spb + (pl.own_fields() ? 0 : rp.cls) + rp.wls;
 }
 
 // Steps of one launch whose rows for nr rings fit the budget.
@@ -802,7 +821,7 @@ static int fill_orders(qa_ctx *ctx, const RingPlan &pl, const RingParams &rp, in
     const long long total = (long long)(rp.step1 - rp.step0) * rp.ord_per_step * n_rings;
     if (total <= 0) return QA_OK;
     const size_t need = order_fill_bytes(pl.n_max);
-    const int with_cls = pl.pm1 || pl.sparse ? 0 : 1;
+    const int with_cls = pl.own_fields() ? 0 : 1;
     if (need <= (size_t)ctx->smem_optin) {
         const int grid = (int)std::min<long long>(total, (long long)ctx->sms * 8);
         QA_TRY(opt_in_smem(ctx, (const void *)order_fill_kernel, need));
@@ -852,6 +871,13 @@ int launch_rings(qa_ctx *ctx, int kind, const RingPlan &pl, RingParams rp, int n
     if (pl.pm1) {
         auto kern = pl.gbytes == 4 ? ring_pm1_kernel<int, true>
                                    : (pl.jw_smem ? ring_pm1_kernel<short, true> : ring_pm1_kernel<short, false>);
+        QA_TRY(opt_in_smem(ctx, (const void *)kern, pl.smem));
+        kern<<<n_rings, 32 * pl.W, pl.smem, strm>>>(rp);
+        QA_CK(cudaGetLastError());
+        return QA_OK;
+    }
+    if (pl.slab) {
+        auto kern = slab_kernel(pl);
         QA_TRY(opt_in_smem(ctx, (const void *)kern, pl.smem));
         kern<<<n_rings, 32 * pl.W, pl.smem, strm>>>(rp);
         QA_CK(cudaGetLastError());
@@ -914,6 +940,20 @@ static int sqa_rot_seg(qa_ctx *ctx, int steps) {
     return rot_seg(ctx, std::max(25, std::min(100, steps / 8)), steps);
 }
 
+// Steps per rotated launch of a PT segment of `range` steps with `sweeps` sweeps
+// a step; 0: too short to rotate.  An eighth of the segment, which has at least
+// 8 sweeps.  ring_slab_kernel's sweeps are short against a launch: at least 6
+// sweeps a launch and two launches (1024 rings, n = 2048, 25 sweeps a step:
+// whole-grid 56.1, rotated 52.3 ms; 2 sweeps a step, segments of 10: whole-grid
+// 18.4, rotated step by step 25.6 ms).
+static int pt_rot_seg(qa_ctx *ctx, const RingPlan &pl, int range, int sweeps) {
+    if ((long long)range * sweeps < 8) return 0;
+    const int seg = rot_seg(ctx, std::max(1, range / 8), range);
+    if (!pl.slab || ctx->tune.rot_steps > 0) return seg;
+    const int need = std::max(seg, (6 + sweeps - 1) / sweeps);
+    return range >= 2 * need ? need : 0;
+}
+
 // Whether nr rings are worth rotating: more rings than SMs, and whole-grid
 // launches would leave more than 3% of the resident slots idle.  With w the
 // number of waves (rings over resident CTAs per SM times SMs), the last of
@@ -934,6 +974,8 @@ static bool rotation_pays(qa_ctx *ctx, int kind, const RingPlan &pl, int nr) {
                                             : (const void *)ring_pm1_kernel<short, false>);
     else if (pl.sparse)
         kern = (const void *)ring_sparse_kernel;
+    else if (pl.slab)
+        kern = (const void *)slab_kernel(pl);
     else if (pl.dense)
         kern = (const void *)dense_kernel(pl);
     else
@@ -990,7 +1032,8 @@ static int plan_models(qa_ctx *ctx, const qa_problem *const *probs, int np, int 
     bool pays = false;
     for (int m = 0; m < np; ++m) {
         QA_TRY(plan_rings(ctx, probs + m, 1, kind, P, probs[m]->n, &mr[m].pl, nr, clusters, ref_order));
-        if (mr[m].pl.pm1 != set_pl.pm1 || mr[m].pl.sparse != set_pl.sparse || mr[m].pl.dense != set_pl.dense)
+        if (mr[m].pl.pm1 != set_pl.pm1 || mr[m].pl.sparse != set_pl.sparse || mr[m].pl.dense != set_pl.dense ||
+            mr[m].pl.slab != set_pl.slab)
             mr[m].pl = set_pl;
         mr[m].g0 = m * (nr / np);
         mr[m].nr = nr / np;
@@ -2748,23 +2791,29 @@ static int sqapt_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_prob
     sp.ring_in = d_rin; sp.slot_of = d_slot; sp.avg_trace = d_avg; sp.swap_trace = d_swp; sp.steps_total = steps;
     QA_CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     int n_seg = 0, n_launch = 0;
-    const bool rotate = rotation_pays(ctx, kind, pl, nr);
-    std::vector<ModelRun> mr;  // an instance set of uneven size: per-model launches
-    if (!rotate)
+    const int sweeps = rp.spb + rp.wls + rp.cls;
+    bool rotate =
+        pt_rot_seg(ctx, pl, std::min(prm->swap_interval, steps), sweeps) > 0 && rotation_pays(ctx, kind, pl, nr);
+    // an instance set of uneven size: per-model launches (slab: also where the set
+    // could rotate, since the small models' rings cost far less shared memory;
+    // 6 models, n = 512 .. 4096, 1536 rings: rotated 54.2, per model 47.6 ms)
+    std::vector<ModelRun> mr;
+    if (!rotate || pl.slab)
         QA_TRY(plan_models(ctx, problems, n_problems, kind, P, pl, nr, prm->cluster_sweeps > 0,
                            !classical && ctx->update_order == QA_ORDER_REFERENCE, &mr));
+    rotate = rotate && mr.empty();
     for (int s0 = 0; s0 < steps;) {
         const int s1 = std::min({steps, (s0 / prm->swap_interval + 1) * prm->swap_interval, s0 + 256});
         rp.step0 = s0;
         rp.step1 = s1;
         rp.init_scan = s0 == 0;
         rp.init_fields = s0 == 0;
-        // at least 8 sweeps in the segment and rings worth rotating: launches
-        // of an eighth of it (at least one step), joined before the swaps
-        if ((long long)(s1 - s0) * (rp.spb + rp.wls + rp.cls) >= 8 && rotate) {
+        // rings worth rotating and a segment long enough: short launches,
+        // joined before the swaps
+        const int seg = rotate ? pt_rot_seg(ctx, pl, s1 - s0, sweeps) : 0;
+        if (seg > 0) {
             int nl = 0;
-            QA_TRY(run_rings_rotated(ctx, kind, pl, rp, nr, s0, s1, rot_seg(ctx, std::max(1, (s1 - s0) / 8), s1 - s0),
-                                         &nl));
+            QA_TRY(run_rings_rotated(ctx, kind, pl, rp, nr, s0, s1, seg, &nl));
             n_launch += nl;
         } else if (!mr.empty()) {
             int nl = 0;

@@ -148,7 +148,9 @@ __device__ __forceinline__ unsigned long long spin_wait(const SpinPipe &pp, int 
 // y >= limit, up to 2e-5 (the approximate log2 is good to 4e-6, e^y's own
 // polynomial and the roundings to about 1e-5).  u = 0 accepts iff y > -17.
 __device__ __forceinline__ float accept_limit(float u24v) {
-    return fmaxf(__fmaf_rn(__log2f(u24v), 0.693147181f, -16.6355323f), -17.0f);
+    float l;
+    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(l) : "f"(u24v));  // u24 is 0 or at least 1
+    return fmaxf(__fmaf_rn(l, 0.693147181f, -16.6355323f), -17.0f);
 }
 // Distance from the limit below which the exact test decides: five times the
 // limit's error, and the rounding of limit + Trotter term where T4 is large.
