@@ -352,8 +352,23 @@ double trotter_coupling(double beta, double gamma, int P) {
 
 std::vector<uint32_t> dummy;
 
+// Packed spins to +-1 bytes, eight at a time by table (a bit at a time took
+// 4.8 ns a spin: 10 ms of a 50 ms SQA-PT call that returns 1056 states of 2048).
+struct SpinBytes {
+    uint64_t of[256];
+    SpinBytes() {
+        for (int b = 0; b < 256; ++b) {
+            int8_t s[8];
+            for (int k = 0; k < 8; ++k) s[k] = (b >> k) & 1 ? 1 : -1;
+            std::memcpy(&of[b], s, 8);
+        }
+    }
+};
 void unpack_bits(const uint32_t *bits, int n, int8_t *out) {
-    for (int i = 0; i < n; ++i) out[i] = ((bits[i >> 5] >> (i & 31)) & 1u) ? 1 : -1;
+    static const SpinBytes table;
+    int i = 0;
+    for (; i + 8 <= n; i += 8) std::memcpy(out + i, &table.of[(bits[i >> 5] >> (i & 31)) & 0xFFu], 8);
+    for (; i < n; ++i) out[i] = ((bits[i >> 5] >> (i & 31)) & 1u) ? 1 : -1;
 }
 
 int check_batch(const qa_problem *const *probs, int np, int *kind, int *n_max) {
