@@ -22,6 +22,7 @@
 #include "qa_tc.cuh"
 #include "qa_pm1.cuh"
 #include "qa_pt.cuh"
+#include "qa_ptc.cuh"
 #include "qa_ingest.cuh"
 #include "qa_dense.cuh"
 #include "qa_slab.cuh"
@@ -2817,7 +2818,23 @@ static int sqapt_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_prob
         QA_TRY(plan_models(ctx, problems, n_problems, kind, P, pl, nr, prm->cluster_sweeps > 0,
                            !classical && ctx->update_order == QA_ORDER_REFERENCE, &mr));
     rotate = rotate && mr.empty();
-    for (int s0 = 0; s0 < steps;) {
+    // classical chains of +-1 models: the whole run in one launch
+    const bool chains = classical && pl.pm1 && Rn <= 32 && ptc_smem_bytes(Rn, n_max) <= (size_t)ctx->smem_optin &&
+                        !std::getenv("QA_DISABLE_PT_CHAINS");
+    if (chains) {
+        PTChainParams cp{};
+        cp.probs = d_probs; cp.rings = d_rings; cp.spins = d_spins; cp.B = d_B; cp.bp = d_bpjp;
+        cp.R = Rn; cp.steps = steps; cp.spb = prm->sweeps_per_step; cp.swap_interval = prm->swap_interval;
+        cp.nw_max = L.nw_max; cp.best_E = d_best; cp.best_step = d_bstep; cp.best_slot = d_bslot;
+        cp.best_bits = d_bits; cp.final_bits = d_fbits; cp.last_E = d_min + steps; cp.rec_stride = steps + 1;
+        cp.ring_in = d_rin; cp.avg_trace = d_avg; cp.swap_trace = d_swp; cp.counters = d_cnt;
+        const size_t sm = ptc_smem_bytes(Rn, n_max);
+        QA_TRY(opt_in_smem(ctx, (const void *)pt_chains_kernel, sm));
+        pt_chains_kernel<<<reads_total, 32 * Rn, sm, ctx->stream>>>(cp);
+        QA_CK(cudaGetLastError());
+        n_launch = 1;
+    }
+    for (int s0 = 0; s0 < steps && !chains;) {
         const int s1 = std::min({steps, (s0 / prm->swap_interval + 1) * prm->swap_interval, s0 + 256});
         rp.step0 = s0;
         rp.step1 = s1;
