@@ -23,6 +23,7 @@
 #include "qa_pm1.cuh"
 #include "qa_pt.cuh"
 #include "qa_ptc.cuh"
+#include "qa_sa.cuh"
 #include "qa_ingest.cuh"
 #include "qa_dense.cuh"
 #include "qa_slab.cuh"
@@ -1792,9 +1793,13 @@ static int sa_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_problem
 
     // dense +-1 couplings: bits and int32 fields in shared memory (fields built in-kernel);
     // traced runs take the generic kernel, which gives the same results
-    bool pm1 = kind == K_DENSE && !traces && sa_pm1_smem_bytes(n_max) <= (size_t)ctx->smem_optin &&
+    bool pm1 = kind == K_DENSE && !traces && sa_dense_smem_bytes<true>(n_max) <= (size_t)ctx->smem_optin &&
                !std::getenv("QA_DISABLE_PM1");
     for (int p = 0; p < n_problems && pm1; ++p) pm1 = problems[p]->dev.Jw != nullptr;
+    // other dense couplings: float32 rows read at each flip
+    bool real = kind == K_DENSE && !traces && !pm1 && sa_dense_smem_bytes<false>(n_max) <= (size_t)ctx->smem_optin &&
+                !std::getenv("QA_DISABLE_DENSE");
+    for (int p = 0; p < n_problems && real; ++p) real = problems[p]->plain_j;
     QA_CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, 1, n_max, L.nw_max, DOM_INIT, !pm1));
     const int nwp = (L.nw_max + 3) & ~3, np4 = (n_max + 3) & ~3;
@@ -1809,11 +1814,11 @@ static int sa_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_problem
     sp.tr_bits = d_trb; sp.tr_E = d_tre; sp.tr_end_bits = d_treb; sp.tr_stride = stride; sp.tr_rps = rps;
     QA_CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     int rc = QA_OK;
-    if (pm1) {
-        const size_t sm1 = sa_pm1_smem_bytes(n_max);
-        if (sm1 > 48 * 1024)
-            QA_CK(cudaFuncSetAttribute(sa_pm1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm1));
-        sa_pm1_kernel<<<nr, 32, sm1, ctx->stream>>>(sp);
+    if (pm1 || real) {
+        auto kern = pm1 ? sa_dense_kernel<true> : sa_dense_kernel<false>;
+        const size_t sm1 = pm1 ? sa_dense_smem_bytes<true>(n_max) : sa_dense_smem_bytes<false>(n_max);
+        QA_TRY(opt_in_smem(ctx, (const void *)kern, sm1));
+        kern<<<nr, 32 * sa_warps(n_max), sm1, ctx->stream>>>(sp);
         QA_CK(cudaGetLastError());
     } else {
         dispatch_kind(kind, [&](auto K) {
