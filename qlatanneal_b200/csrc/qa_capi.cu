@@ -24,6 +24,7 @@
 #include "qa_pt.cuh"
 #include "qa_ptc.cuh"
 #include "qa_sa.cuh"
+#include "qa_hubo.cuh"
 #include "qa_ingest.cuh"
 #include "qa_dense.cuh"
 #include "qa_slab.cuh"
@@ -643,6 +644,7 @@ struct RingPlan {
     bool sparse = false;  // ring_sparse_kernel
     bool dense = false;   // ring_dense_kernel
     bool slab = false;    // ring_slab_kernel
+    bool hubo = false;    // ring_hubo_kernel
     bool wide = false;    // slab: 64-bit worldline words (P > 32)
     bool own_fields() const { return pm1 || sparse || slab; }  // no field cache to initialise
     int gbytes = 4;       // pm1: bytes per field (4 int32, 2 int16)
@@ -740,6 +742,16 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
         // 600 rings: n = 24 23.3 -> 17.7 ms, n = 64 36.8 -> 28.3, n = 200
         // 69.9 -> 66.4; 300 rings of n = 900 25.1 -> 28.2, so not there)
         if (ctx->tune.warps_per_ring <= 0) pl->W = std::min(P, n_rings >= 2 * ctx->sms && n_max <= 256 ? 8 : 16);
+        pl->W = std::min(pl->W, 16);
+        return QA_OK;
+    }
+    // terms of at most four spins: ring_hubo_kernel
+    pl->hubo = !clusters && kind == K_HUBO && P <= 64 && !std::getenv("QA_DISABLE_HUBO") &&
+               hubo_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin;
+    for (int p = 0; p < np && pl->hubo; ++p) pl->hubo = probs[p]->dev.hub_rec != nullptr;
+    if (pl->hubo) {
+        pl->smem = hubo_smem_bytes(P, n_max, ref_order);
+        if (ctx->tune.warps_per_ring <= 0) pl->W = std::min(P, 16);
         pl->W = std::min(pl->W, 16);
         return QA_OK;
     }
@@ -893,6 +905,13 @@ int launch_rings(qa_ctx *ctx, int kind, const RingPlan &pl, RingParams rp, int n
         QA_CK(cudaGetLastError());
         return QA_OK;
     }
+    if (pl.hubo) {
+        auto kern = pl.ref_order ? ring_hubo_kernel<true> : ring_hubo_kernel<false>;
+        QA_TRY(opt_in_smem(ctx, (const void *)kern, pl.smem));
+        kern<<<n_rings, 32 * pl.W, pl.smem, strm>>>(rp);
+        QA_CK(cudaGetLastError());
+        return QA_OK;
+    }
     if (pl.slab) {
         auto kern = slab_kernel(pl);
         QA_TRY(opt_in_smem(ctx, (const void *)kern, pl.smem));
@@ -991,6 +1010,8 @@ static bool rotation_pays(qa_ctx *ctx, int kind, const RingPlan &pl, int nr) {
                                             : (const void *)ring_pm1_kernel<short, false>);
     else if (pl.sparse)
         kern = (const void *)ring_sparse_kernel;
+    else if (pl.hubo)
+        kern = pl.ref_order ? (const void *)ring_hubo_kernel<true> : (const void *)ring_hubo_kernel<false>;
     else if (pl.slab)
         kern = (const void *)slab_kernel(pl);
     else if (pl.dense)
@@ -1050,7 +1071,7 @@ static int plan_models(qa_ctx *ctx, const qa_problem *const *probs, int np, int 
     for (int m = 0; m < np; ++m) {
         QA_TRY(plan_rings(ctx, probs + m, 1, kind, P, probs[m]->n, &mr[m].pl, nr, clusters, ref_order));
         if (mr[m].pl.pm1 != set_pl.pm1 || mr[m].pl.sparse != set_pl.sparse || mr[m].pl.dense != set_pl.dense ||
-            mr[m].pl.slab != set_pl.slab)
+            mr[m].pl.slab != set_pl.slab || mr[m].pl.hubo != set_pl.hubo)
             mr[m].pl = set_pl;
         mr[m].g0 = m * (nr / np);
         mr[m].nr = nr / np;
@@ -1572,10 +1593,11 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
     // flip updates grouped by target (terms of degree <= 4 only)
     bool small_terms = true;
     for (int t = 0; t < n_terms && small_terms; ++t) small_terms = tptr[t + 1] - tptr[t] <= 4;
-    std::vector<int> upd_ptr, upd_run;
-    std::vector<int4> upd_rec;
+    std::vector<int> hub_ptr;
+    std::vector<int4> hub_rec;
     if (small_terms) {
-        upd_ptr.assign(n + 1, 0);
+        hub_ptr.assign(n + 1, 0);
+        std::vector<std::vector<int4>> layer;  // layer k: the k-th record of each target
         struct U { int v, t, w1, w2; };
         std::vector<U> u;
         for (int j = 0; j < n; ++j) {
@@ -1592,16 +1614,21 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
                 }
             }
             std::stable_sort(u.begin(), u.end(), [](const U &a, const U &b) { return a.v != b.v ? a.v < b.v : a.t < b.t; });
-            for (size_t k = 0; k < u.size(); ++k) {
-                if (k == 0 || u[k].v != u[k - 1].v) upd_run.push_back((int)upd_rec.size());
+            layer.clear();
+            for (size_t k = 0, l = 0; k < u.size(); ++k) {
+                l = k > 0 && u[k].v == u[k - 1].v ? l + 1 : 0;
+                if (layer.size() <= l) layer.emplace_back();
                 const float two = 2.0f * c32[u[k].t];
                 int bits;
                 std::memcpy(&bits, &two, 4);
-                upd_rec.push_back(make_int4(u[k].v, u[k].w1, u[k].w2, bits));
+                layer[l].push_back(make_int4(u[k].v, u[k].w1, u[k].w2, bits));
             }
-            upd_ptr[j + 1] = (int)upd_run.size();
+            for (auto &l : layer) {
+                l.resize((l.size() + 31) / 32 * 32, make_int4(-1, -1, -1, 0));
+                hub_rec.insert(hub_rec.end(), l.begin(), l.end());
+            }
+            hub_ptr[j + 1] = (int)(hub_rec.size() / 32);
         }
-        upd_run.push_back((int)upd_rec.size());
     }
     qa_problem *P = new qa_problem();
     P->ctx = ctx;
@@ -1618,9 +1645,8 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
     if (rc == QA_OK) rc = upload(P, c32.data(), c32.size(), &P->dev.coef32);
     if (rc == QA_OK) rc = upload(P, coeff, (size_t)n_terms, &P->dev.coef64);
     if (rc == QA_OK && small_terms) {
-        rc = upload(P, upd_ptr.data(), upd_ptr.size(), &P->dev.upd_ptr);
-        if (rc == QA_OK) rc = upload(P, upd_run.data(), upd_run.size(), &P->dev.upd_run);
-        if (rc == QA_OK) rc = upload(P, upd_rec.data(), upd_rec.size(), &P->dev.upd_rec);
+        rc = upload(P, hub_ptr.data(), hub_ptr.size(), &P->dev.hub_ptr);
+        if (rc == QA_OK) rc = upload(P, hub_rec.data(), hub_rec.size(), &P->dev.hub_rec);
         // one 16-byte record per term for the per-step energy scan
         std::vector<int4> trec(std::max(n_terms, 1), make_int4(-1, -1, -1, -1));
         for (int t = 0; t < n_terms; ++t) {

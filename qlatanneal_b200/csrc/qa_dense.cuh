@@ -344,11 +344,11 @@ __device__ __noinline__ int dense_worldlines(const float *J, uint32_t ordo, int 
                 if (x + 32 * k < n32) uw[x + 32 * k] = u24(pick(r, k));
         }
     __syncthreads();
-    int moves = 0;
+    int moves = 0, look = W;  // blocks of a round: two after one with moves, else all warps'
     uint32_t *mk = mask;
     for (int q0 = 0; q0 < nw;) {
         // this round: warp w evaluates block q0 + w on the current state
-        const int q = q0 + warp, pos = (q << 5) | lane;
+        const int q = warp < look ? q0 + warp : nw, pos = (q << 5) | lane;
         const bool valid = q < nw && pos < n;
         const int i = !valid ? 0 : (ORD ? (int)dsm<OrdT>(ordo)[pos] : pos);
         const unsigned long long wi = Wc[i];
@@ -371,9 +371,11 @@ __device__ __noinline__ int dense_worldlines(const float *J, uint32_t ordo, int 
         const uint32_t with = __ballot_sync(FULL, lane < W && mk[lane] != 0u);
         mk = mk == mask ? mask + 32 : mask;
         if (!with) {
-            q0 += W;
+            q0 += look;
+            look = W;
             continue;
         }
+        look = min(2, W);
         const int ws = __ffs(with) - 1;
         if (warp == ws) {
             // resolve the block in position order on a copy of its fields

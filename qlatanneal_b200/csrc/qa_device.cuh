@@ -151,12 +151,13 @@ struct ProbDev {
     // bits J[m][32q .. 32q+31] (1 = +1; diagonal and padding bits 0); else null
     const uint32_t *Jw;
     // hubo with every term of degree <= 4: the field updates of a flip of
-    // spin j grouped by target.  Runs upd_run[upd_ptr[j] .. upd_ptr[j+1]) of
-    // j; run r = records upd_rec[upd_run[r] .. upd_run[r+1]), one target v,
-    // its terms in increasing term order; record = {v, w1, w2, bits(2 J_t)}
-    // with w1, w2 the term's other spins (-1: none).  Else null.
-    const int *upd_ptr, *upd_run;
-    const int4 *upd_rec;
+    // spin j in chunks hub_ptr[j] .. hub_ptr[j+1] of 32 records (one load of a
+    // warp), hub_rec[32 c + lane] = {v, w1, w2, bits(2 J_t)}: target v (-1: no
+    // record), w1, w2 the term's other spins (-1: none).  A chunk holds a target
+    // once; a target's terms stand in increasing order, one chunk after another.
+    // Else null.
+    const int *hub_ptr;
+    const int4 *hub_rec;
     // hubo with every term of degree <= 4: term t's spins {v0, v1, v2, v3}
     // (-1: none) in one 16-byte record, for the per-step energy scan; else null
     const int4 *trec;
@@ -189,15 +190,15 @@ __device__ __forceinline__ void apply_flip(const ProbDev &P, float *g, const uin
             const int m = __ldg(P.col + e);
             g[m] = __fadd_rn(g[m], __fmul_rn(cf, __ldg(P.val32 + e)));
         }
-    } else if (P.upd_rec) {
+    } else if (P.hub_rec) {
         // one lane per target spin v, its terms in order: the same float
         // additions, in the same order per field, as the term-by-term loop
         const int sj = spin_of(S, j);  // S holds the new spin
-        const int r0 = __ldg(P.upd_ptr + j), r1 = __ldg(P.upd_ptr + j + 1);
-        for (int r = r0 + lane; r < r1; r += 32) {
-            const int a = __ldg(P.upd_run + r), b = __ldg(P.upd_run + r + 1);
-            for (int k = a; k < b; ++k) {
-                const int4 rc = __ldg(P.upd_rec + k);
+        const int a = __ldg(P.hub_ptr + j), b = __ldg(P.hub_ptr + j + 1);
+        for (int c = a; c < b; ++c) {
+            const int4 rc = __ldg(P.hub_rec + 32 * c + lane);
+            if (c > a) __syncwarp();
+            if (rc.x >= 0) {
                 int pr = sj;
                 if (rc.y >= 0) pr *= spin_of(S, rc.y);
                 if (rc.z >= 0) pr *= spin_of(S, rc.z);

@@ -1,0 +1,444 @@
+// qa_hubo.cuh -- Trotter-ring sweep kernel for higher-order models whose terms
+// have at most four spins.
+//
+// Same replay semantics as ring_kernel<K_HUBO>.  What bounds this path is the
+// chain of an accepted flip: its field updates, and the decisions after it.
+//  * a flip's updates are 32-record chunks (ProbDev::hub_rec), one coalesced load
+//    for the warp, asked for while the flip before is applied;
+//  * after a flip only lanes whose field it changed decide again (the inverse
+//    order tells which of the updated spins sit in the block);
+//  * worldline moves: a warp evaluates a block of 32 positions, the moves before
+//    the first lane that one of them changes are applied to all slices together,
+//    and the evaluation resumes at that lane;
+//  * the energy scan takes a term's sign in every slice from the xor of its
+//    spins' worldline words.
+// n = 1024, P = 16, 128 reads, 60 steps: slice sweeps alone 16.2 -> 8.8 ms, with
+// one worldline sweep a step 33.8 -> 17.3 ms.  What is left is about 150
+// instructions a flip at 1.6 a cycle, and in the worldline sweeps the barriers of
+// a round per block.  Not kept: the chunks of all lanes that will flip prefetched
+// ahead of the wait for the previous slice (8.8 -> 8.9 ms).
+#pragma once
+#include "qa_slab.cuh"
+
+namespace qa {
+
+struct HuboLay {
+    uint32_t G, S, W, h, uw, inv, ord0, ord1, prog, abortf, cellE, part, mask, wsp, flag, total;
+};
+__host__ __device__ inline HuboLay hubo_layout(int P, int n, bool ref_order) {
+    const int nw = (n + 31) / 32, n32 = nw * 32, ld = dense_ld(n);
+    HuboLay L{};
+    uint32_t o = 0;
+    auto take = [&](size_t bytes) {
+        const uint32_t at = o;
+        o += (uint32_t)align_up(bytes, 16);
+        return at;
+    };
+    L.G = take((size_t)P * ld * 4);
+    L.S = take((size_t)P * nw * 4);
+    L.W = take((size_t)n32 * 8);     // worldline words, built for the energy scan
+    L.h = take((size_t)n32 * 4);
+    L.uw = take((size_t)n32 * 4);    // worldline uniforms
+    L.cellE = take((size_t)P * 8);
+    L.part = take(32 * 4);
+    L.mask = take(2 * 32 * 4);       // move masks of a worldline round, two rounds
+    L.wsp = take(32 * 4);            // a worldline batch's spins
+    L.flag = take(16);               // [0]: best slice, [1]: batch, [2]: first lane to decide again, [3]: lowest slice
+    L.prog = take((size_t)P * 4);
+    L.abortf = take(4);
+    if (ref_order) {
+        L.inv = take((size_t)n32 * 2);
+        L.ord0 = take(ord_row_bytes(n32));
+        L.ord1 = take(ord_row_bytes(n32));
+    }
+    L.total = o;
+    return L;
+}
+__host__ __device__ inline size_t hubo_smem_bytes(int P, int n, bool ref_order) {
+    return hubo_layout(P, n, ref_order).total;
+}
+
+// One record's update after a flip of its spin (new value sj = +-1): S holds the
+// flip.
+__device__ __forceinline__ void hubo_add(const int4 &r, float *g, const uint32_t *S, int sj) {
+    if (r.x < 0) return;
+    uint32_t down = sj < 0 ? 1u : 0u;
+    if (r.y >= 0) down ^= down_bit(S, r.y);
+    if (r.z >= 0) down ^= down_bit(S, r.z);
+    const float two = __int_as_float(r.w);
+    g[r.x] = __fadd_rn(g[r.x], down ? -two : two);
+}
+
+// The lanes of block q (positions) that hold record r's target.
+template <bool ORD>
+__device__ __forceinline__ uint32_t hubo_touch(const int4 &r, const OrdT *inv, int q) {
+    if (r.x < 0) return 0u;
+    const int p = ORD ? (int)inv[r.x] : r.x;
+    return (p >> 5) == q ? 1u << (p & 31) : 0u;
+}
+
+// Slices t0, t0 + dt, .. < t1 of one slice sweep, one warp; the number of flips.
+template <bool ORD>
+__device__ __noinline__ int hubo_sweep(const int *hptr, const int4 *hrec, uint32_t ordo, unsigned long long *err, int n,
+                                       int NP, int t0, int t1, int dt, float B, float T4, uint64_t key, uint32_t cell,
+                                       uint32_t sigma, uint32_t tag) {
+    const int lane = threadIdx.x & 31, nw = (n + 31) >> 5, ld = dense_ld(n);
+    const HuboLay L = hubo_layout(NP, n, ORD);
+    uint32_t *S = dsm<uint32_t>(L.S);
+    const float *h = dsm<float>(L.h);
+    const OrdT *ord = dsm<OrdT>(ordo), *inv = dsm<OrdT>(L.inv);
+    int *prog = dsm<int>(L.prog), *abortf = dsm<int>(L.abortf);
+    const float eps = accept_margin(T4);
+    int flips = 0;
+    for (int t = t0; t < t1; t += dt) {
+        const int tp = t == 0 ? NP - 1 : t - 1, tn = t + 1 == NP ? 0 : t + 1;
+        uint32_t *St = S + t * nw;
+        const uint32_t *Sp = S + tp * nw, *Sn = S + tn * nw;
+        float *gt = dsm<float>(L.G) + t * ld;
+        U4 r{0, 0, 0, 0};
+#pragma unroll 1
+        for (int q = 0; q < nw; ++q) {
+            if ((q & 3) == 0) r = philox((uint32_t)(((q >> 2) << 5) | lane), cell + (uint32_t)t, sigma, tag, key);
+            const int pos = (q << 5) | lane;
+            const bool valid = pos < n;
+            const int i = valid ? (ORD ? (int)ord[pos] : pos) : 0;
+            const int c0 = __ldg(hptr + i), c1 = __ldg(hptr + i + 1);  // the spin's chunks
+            const float u = u24(pick(r, q & 3)), hi = h[i];
+            const uint32_t sb = (St[i >> 5] >> (i & 31)) & 1u;
+            const float Bs = sb ? B : -B, lim0 = accept_limit(u);
+            float gi = gt[i];
+            if (ORD && t > 0) {
+                slab_wait(prog + t - 1, q + 1, abortf, err, lane);
+                if (tn == 0) slab_wait(prog, q + 1, abortf, err, lane);
+            }
+            const int d = (int)(((Sp[i >> 5] >> (i & 31)) & 1u) ^ sb) + (int)(((Sn[i >> 5] >> (i & 31)) & 1u) ^ sb);
+            const float tro = __fmul_rn(__int2float_rn(1 - d), T4), lim = lim0 + tro;
+            auto decide = [&]() {
+                const float xs = __fmul_rn(__fadd_rn(hi, gi), Bs);
+                bool ok = xs >= lim;
+                if (__any_sync(FULL, !(fabsf(xs - lim) > eps))) ok = metropolis_nb24(__fsub_rn(xs, tro), u);
+                return __ballot_sync(FULL, valid & ok);
+            };
+            uint32_t m = decide();
+            if (m) {
+                auto chunk = [&](int j) {  // the first chunk of lane j's spin (nothing when it has none)
+                    const int a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
+                    return a < b ? __ldg(hrec + 32 * a + lane) : make_int4(-1, -1, -1, 0);
+                };
+                int j = __ffs(m) - 1;
+                int4 rec = chunk(j);
+                while (true) {
+                    const uint32_t pend = j == 31 ? 0u : ~((2u << j) - 1u);
+                    const int jj = __shfl_sync(FULL, i, j), a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
+                    const int sj = __shfl_sync(FULL, sb, j) ? -1 : 1;  // the new spin
+                    if (lane == 0) St[jj >> 5] ^= 1u << (jj & 31);
+                    ++flips;
+                    const int jn = (m & pend) ? __ffs(m & pend) - 1 : j;  // the likely next flip
+                    const int4 recn = chunk(jn);
+                    __syncwarp();
+                    hubo_add(rec, gt, St, sj);
+                    uint32_t touch = hubo_touch<ORD>(rec, inv, q);
+                    for (int c = a + 1; c < b; ++c) {  // (chunks in order: a target's terms stay in order)
+                        const int4 x = __ldg(hrec + 32 * c + lane);
+                        __syncwarp();
+                        hubo_add(x, gt, St, sj);
+                        touch |= hubo_touch<ORD>(x, inv, q);
+                    }
+                    touch = __reduce_or_sync(FULL, touch) & pend;
+                    __syncwarp();
+                    if (touch) {
+                        if ((touch >> lane) & 1u) gi = gt[i];
+                        m = (m & ~touch) | (decide() & touch);
+                    }
+                    if (!(m & pend)) break;
+                    const int k = __ffs(m & pend) - 1;
+                    rec = k == jn ? recn : chunk(k);
+                    j = k;
+                }
+            }
+            if (ORD) {
+                __threadfence_block();
+                __syncwarp();
+                if (lane == 0) st_release_cta(prog + t, q + 1);
+            }
+        }
+    }
+    return flips;
+}
+
+// One worldline sweep, whole CTA (ends with a barrier); the number of moves.
+template <bool ORD>
+__device__ __noinline__ int hubo_worldlines(const int *hptr, const int4 *hrec, uint32_t ordo, int n, int NP, float B,
+                                            uint64_t key, uint32_t slot, uint32_t sigma) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
+    const int nw = (n + 31) >> 5, n32 = nw * 32, ld = dense_ld(n);
+    const HuboLay L = hubo_layout(NP, n, ORD);
+    uint32_t *S = dsm<uint32_t>(L.S), *mask = dsm<uint32_t>(L.mask);
+    float *G = dsm<float>(L.G), *uw = dsm<float>(L.uw);
+    const OrdT *ord = dsm<OrdT>(ordo), *inv = dsm<OrdT>(L.inv);
+    int *flag = dsm<int>(L.flag), *wsp = dsm<int>(L.wsp);
+    for (int x = threadIdx.x; x < n32; x += blockDim.x)
+        if (((x >> 5) & 3) == 0) {  // positions q*32 + lane .. + 96: one Philox call
+            const U4 r = philox((uint32_t)(((x >> 7) << 5) | lane), slot, sigma, DOM_WORLD, key);
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+                if (x + 32 * k < n32) uw[x + 32 * k] = u24(pick(r, k));
+        }
+    __syncthreads();
+    int moves = 0, first = 0;  // lanes of block q0 before `first` are done
+    int look = W;              // blocks of a round: two after one with moves, else all warps'
+    uint32_t *mk = mask;
+    for (int q0 = 0; q0 < nw;) {
+        // this round: warp w evaluates block q0 + w on the current state
+        const int q = warp < look ? q0 + warp : nw, pos = (q << 5) | lane;
+        const bool valid = q < nw && pos < n && (warp > 0 || lane >= first);
+        const int i = valid ? (ORD ? (int)ord[pos] : pos) : 0;
+        uint32_t m = 0;
+        if (q < nw) {
+            double Gt = 0.0;
+            int sh = 0;
+            const uint32_t *Sw = S + (i >> 5);
+#pragma unroll 4
+            for (int t = 0; t < NP; ++t) {
+                const uint32_t up = (Sw[t * nw] >> (i & 31)) & 1u;
+                sh += up ? 1 : -1;
+                Gt = __dadd_rn(Gt, (double)signed_by_bit(G[t * ld + i], up));
+            }
+            const float x = __double2float_rn(__dadd_rn(__dmul_rn((double)dsm<float>(L.h)[i], (double)sh), Gt));
+            m = __ballot_sync(FULL, valid & metropolis_nb24(__fmul_rn(x, B), valid ? uw[pos] : 0.0f));
+        }
+        if (lane == 0) mk[warp] = m;
+        __syncthreads();
+        const uint32_t with = __ballot_sync(FULL, lane < W && mk[lane] != 0u);
+        mk = mk == mask ? mask + 32 : mask;
+        if (!with) {
+            q0 += look;
+            look = W;
+            first = 0;
+            continue;
+        }
+        look = min(2, W);
+        const int ws = __ffs(with) - 1;
+        if (warp == ws) {
+            // the moves before the first lane that one of them changes
+            const int c0 = __ldg(hptr + i), c1 = __ldg(hptr + i + 1);
+            uint32_t F = 0, T = 0;
+            for (uint32_t mm = m; mm; mm &= mm - 1u) {
+                const int j = __ffs(mm) - 1;
+                if (T && __ffs(T) - 1 <= j) break;
+                F |= 1u << j;
+                const int a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
+                uint32_t touch = 0;
+                for (int c = a; c < b; ++c) touch |= hubo_touch<ORD>(__ldg(hrec + 32 * c + lane), inv, q);
+                T |= __reduce_or_sync(FULL, touch) & (j == 31 ? 0u : ~((2u << j) - 1u));
+            }
+            wsp[lane] = i;
+            if (lane == 0) {
+                flag[1] = (int)F;
+                flag[2] = T ? __ffs(T) - 1 : 32;
+            }
+        }
+        __syncthreads();
+        const uint32_t F = (uint32_t)flag[1];
+        const int again = flag[2], isp = wsp[lane];
+        const int c0 = __ldg(hptr + isp), c1 = __ldg(hptr + isp + 1);
+        for (int t = warp; t < NP; t += W) {
+            uint32_t *St = S + t * nw;
+            for (uint32_t f = F; f; f &= f - 1u) {
+                const int j = __ffs(f) - 1, jj = __shfl_sync(FULL, isp, j);
+                const int a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
+                const int sj = -spin_of(St, jj);
+                __syncwarp();
+                if (lane == 0) St[jj >> 5] ^= 1u << (jj & 31);
+                for (int c = a; c < b; ++c) {
+                    const int4 x = __ldg(hrec + 32 * c + lane);
+                    __syncwarp();
+                    hubo_add(x, G + t * ld, St, sj);
+                }
+                __syncwarp();
+            }
+        }
+        moves += __popc(F);
+        __syncthreads();
+        q0 += ws;
+        first = again;
+        if (again == 32) {
+            ++q0;
+            first = 0;
+        }
+    }
+    return moves;
+}
+
+// ORD: qanneal's update order.
+template <bool ORD>
+__global__ void __launch_bounds__(512, 1) ring_hubo_kernel(RingParams p) {
+    const RingDev R = p.rings[blockIdx.x];
+    const ProbDev *Pd = p.probs + R.prob;
+    const int NP = p.P, W = p.W, n = Pd->n, nw = Pd->nw, n32 = nw * 32, ld = dense_ld(n), T = Pd->T;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int *hptr = Pd->hub_ptr;
+    const int4 *hrec = Pd->hub_rec;
+    const HuboLay L = hubo_layout(NP, n, ORD);
+    float *G = dsm<float>(L.G), *h = dsm<float>(L.h);
+    uint32_t *S = dsm<uint32_t>(L.S);
+    unsigned long long *Wc = dsm<unsigned long long>(L.W);
+    double *cellE = dsm<double>(L.cellE);
+    int *wpart = dsm<int>(L.part), *flag = dsm<int>(L.flag);
+    if (threadIdx.x == 0) *dsm<int>(L.abortf) = 0;
+    float *Gg = p.fields + R.field_off;
+    for (int t = warp; t < NP; t += W)
+        for (int m = lane; m < n; m += 32) G[t * ld + m] = Gg[(long long)t * n + m];
+    for (int idx = threadIdx.x; idx < NP * nw; idx += blockDim.x) S[idx] = p.spins[R.spin_off + idx];
+    for (int i = threadIdx.x; i < n32; i += blockDim.x) h[i] = i < n ? Pd->h32[i] : 0.0f;
+    __syncthreads();
+
+    const int slot = p.slot ? p.slot[blockIdx.x] : R.k;
+    OrderFeed feed = feed_open(ORD ? dsm<OrdT>(L.ord0) : nullptr, ORD ? dsm<OrdT>(L.ord1) : nullptr,
+                               ORD ? p.ordg + blockIdx.x * p.ord_ring : nullptr, p.ord_stride, n,
+                               ORD ? (p.step1 - p.step0) * p.ord_per_step : 0);
+    unsigned long long att_s = 0, acc_s = 0, att_w = 0, acc_w = 0;
+    double bestE = p.best_E[blockIdx.x];
+    int bestStep = p.best_step[blockIdx.x];
+    // a sweep's order and its inverse, clean progress; whole CTA
+    auto begin_sweep = [&]() {
+        uint32_t ord = 0;
+        for (int t = threadIdx.x; t < NP; t += blockDim.x) dsm<int>(L.prog)[t] = 0;
+        if (ORD) {
+            const OrdT *o = feed_take(feed);
+            OrdT *inv = dsm<OrdT>(L.inv);
+            for (int x = threadIdx.x; x < n; x += blockDim.x) inv[o[x]] = (OrdT)x;
+            ord = (uint32_t)(reinterpret_cast<const unsigned char *>(o) - dense_sm);
+        }
+        __syncthreads();
+        return ord;
+    };
+
+    for (int step = p.step0 - (p.init_scan ? 1 : 0); step < p.step1; ++step) {
+        // step -1 (init_scan) only scores the starting state
+        const int spb = step >= 0 ? p.spb : 0, wls = step >= 0 ? p.wls : 0;
+        const int si_tab = R.sched + (p.per_slot_sched ? slot + max(step, 0) * p.slot_step : max(step, 0));
+        const float B = p.B[si_tab], T4 = p.T4[si_tab];
+        for (int sw = 0; sw < spb; ++sw) {
+            const uint32_t sigma = (uint32_t)(step * p.spb + sw), tag = p.slice_tag | R.tag_extra;
+            const uint32_t ord = begin_sweep();
+            if (ORD) {
+                acc_s += (unsigned long long)hubo_sweep<true>(hptr, hrec, ord, p.counters + 4, n, NP, warp, NP, W, B, T4,
+                                                              R.key, (uint32_t)(slot * NP), sigma, tag);
+                __syncthreads();
+            } else {
+                for (int ph = 0; ph < 3; ++ph) {
+                    const int cnt = phase_count(NP, ph), b = phase_slice(NP, ph, 0);
+                    acc_s += (unsigned long long)hubo_sweep<false>(hptr, hrec, 0, nullptr, n, NP, b + 2 * warp,
+                                                                   b + 2 * cnt, 2 * W, B, T4, R.key,
+                                                                   (uint32_t)(slot * NP), sigma, tag);
+                    if (cnt) __syncthreads();
+                }
+            }
+            if (threadIdx.x == 0) att_s += (unsigned long long)NP * (unsigned long long)n;
+            if (p.mag) {
+                int ps = 0;
+                for (int idx = threadIdx.x; idx < NP * nw; idx += blockDim.x) ps += __popc(S[idx]);
+                ps = warp_sum_i(ps);
+                if (lane == 0) wpart[warp] = ps;
+                __syncthreads();
+                if (threadIdx.x == 0) {
+                    long long tot = 0;
+                    for (int w = 0; w < W; ++w) tot += wpart[w];
+                    p.mag[(long long)blockIdx.x * (p.steps_total * p.spb) + sigma] = (int)(2 * tot - (long long)NP * n);
+                }
+                __syncthreads();
+            }
+            if (p.bsamp) record_bond_sample(p, S, NP, nw, n, wpart, W, step, sw);
+        }
+        for (int sw = 0; sw < wls; ++sw) {
+            const uint32_t sigma = (uint32_t)(step * p.wls + sw);
+            const uint32_t ord = begin_sweep();
+            const int mv = hubo_worldlines<ORD>(hptr, hrec, ord, n, NP, B, R.key, (uint32_t)slot, sigma);
+            if (threadIdx.x == 0) {
+                att_w += (unsigned long long)n;
+                acc_w += (unsigned long long)mv;
+            }
+            __syncthreads();
+        }
+        // ---- step end: slice energies E = c + (sum s h + sum_t J_t prod s), ring sum, best
+        for (int i = threadIdx.x; i < n32; i += blockDim.x) {
+            unsigned long long w = 0;
+            for (int t = 0; t < NP; ++t) w |= (unsigned long long)((S[t * nw + (i >> 5)] >> (i & 31)) & 1u) << t;
+            Wc[i] = ~w;  // down spins
+        }
+        __syncthreads();
+        // slices t and t + 1 of a warp in one pass over the terms, each slice's
+        // sums in cell_energy's order
+        for (int t = 2 * warp; t < NP; t += 2 * W) {
+            double ha = 0.0, hb = 0.0, ja = 0.0, jb = 0.0;
+            for (int i = lane; i < n; i += 32) {
+                const double hv = (double)h[i];
+                const uint32_t w = (uint32_t)(Wc[i] >> t);
+                ha = __dadd_rn(ha, neg_by_bit(hv, w, 0));
+                hb = __dadd_rn(hb, neg_by_bit(hv, w, 1));
+            }
+            for (int k = lane; k < T; k += 32) {
+                const int4 r = __ldg(Pd->trec + k);
+                const double v = (double)__ldg(Pd->coef32 + k);
+                unsigned long long w = Wc[r.x] ^ Wc[r.y];
+                if (r.z >= 0) w ^= Wc[r.z];
+                if (r.w >= 0) w ^= Wc[r.w];
+                const uint32_t b = (uint32_t)(w >> t);
+                ja = __dadd_rn(ja, neg_by_bit(v, b, 0));
+                jb = __dadd_rn(jb, neg_by_bit(v, b, 1));
+            }
+            ha = warp_sum_d(ha);
+            hb = warp_sum_d(hb);
+            ja = warp_sum_d(ja);
+            jb = warp_sum_d(jb);
+            if (lane == 0) {
+                cellE[t] = __dadd_rn(Pd->c, __dadd_rn(ha, ja));
+                if (t + 1 < NP) cellE[t + 1] = __dadd_rn(Pd->c, __dadd_rn(hb, jb));
+            }
+        }
+        const long long bsum = p.ring_bond ? ring_bond_total(S, NP, nw, n, wpart, W) : 0;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            double sum = 0.0, emin = __longlong_as_double(0x7ff0000000000000LL);
+            int tmin = 0;
+            for (int t = 0; t < NP; ++t) {
+                const double E = cellE[t];
+                sum = __dadd_rn(sum, E);
+                if (E < emin) { emin = E; tmin = t; }
+            }
+            const long long ro = (long long)blockIdx.x * p.rec_stride + p.rec_base + step;
+            if (p.ring_sum) p.ring_sum[ro] = sum;
+            if (p.ring_min) p.ring_min[ro] = emin;
+            if (p.ring_bond) p.ring_bond[ro] = bsum;
+            flag[0] = emin < bestE ? tmin : -1;
+            flag[3] = tmin;
+        }
+        __syncthreads();
+        const int tb = flag[0], tl = flag[3];
+        if (tb >= 0) {
+            bestE = cellE[tb];
+            bestStep = step;
+            if (threadIdx.x == 0 && p.best_slot) p.best_slot[blockIdx.x] = slot;
+            for (int q = threadIdx.x; q < nw; q += blockDim.x)
+                p.best_bits[(long long)blockIdx.x * p.nw_max + q] = S[tb * nw + q];
+        }
+        if (p.final_bits && step == p.steps_total - 1)
+            for (int q = threadIdx.x; q < nw; q += blockDim.x)
+                p.final_bits[(long long)blockIdx.x * p.nw_max + q] = S[tl * nw + q];
+        __syncthreads();
+    }
+    for (int idx = threadIdx.x; idx < NP * nw; idx += blockDim.x) p.spins[R.spin_off + idx] = S[idx];
+    for (int t = warp; t < NP; t += W)
+        for (int m = lane; m < n; m += 32) Gg[(long long)t * n + m] = G[t * ld + m];
+    if (lane == 0) atomicAdd(p.counters + 1, acc_s);
+    if (threadIdx.x == 0) {
+        atomicAdd(p.counters + 0, att_s);
+        atomicAdd(p.counters + 2, att_w);
+        atomicAdd(p.counters + 3, acc_w);
+        p.best_E[blockIdx.x] = bestE;
+        p.best_step[blockIdx.x] = bestStep;
+    }
+}
+
+}  // namespace qa
