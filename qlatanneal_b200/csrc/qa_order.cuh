@@ -248,7 +248,11 @@ __device__ __forceinline__ void pipe_publish(const SlicePipe &pp, int t, int q, 
         __threadfence_block();
         __syncwarp();
     }
-    st_release_cta(pp.prog + t, q + 1);
+    if (fenced)
+        st_release_cta(pp.prog + t, q + 1);
+    else  // the warp has written nothing since its last fence, which orders what came before
+        asm volatile("st.relaxed.cta.shared.b32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(pp.prog + t)), "r"(q + 1)
+                     : "memory");
 }
 
 }  // namespace qa

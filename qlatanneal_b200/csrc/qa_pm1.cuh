@@ -216,7 +216,7 @@ __device__ __forceinline__ void pm1_block_ord(const uint32_t *Jw, uint32_t *St, 
         const float xs = __fmul_rn(signed_by_bit(hg, sb), B);
         const float ya = __fsub_rn(xs, __fmul_rn(__int2float_rn(1 - dn), T4));
         const float yb = __fsub_rn(xs, __fmul_rn(__int2float_rn(-dn), T4));
-        if (!__any_sync(FULL, valid & (metropolis_maybe24(ya, u) | metropolis_maybe24(yb, u)))) {
+        if (!__any_sync(FULL, valid & metropolis_maybe24(fmaxf(ya, yb), u))) {  // (the test is monotone in y)
             pipe_publish(pp, t, q, lane, false);  // no flips in the block, nothing written
             return;
         }
