@@ -266,6 +266,23 @@ __device__ __forceinline__ float pm1_world_y(float hi, unsigned long long wi, in
     return __fmul_rn(__double2float_rn(__dadd_rn(__dmul_rn((double)hi, (double)sh), (double)gs)), B);
 }
 
+// Slice sum sum_t s_t,i g_t,i of spin i (g: its fields, a slice every npad) by its
+// worldline word.
+template <typename GT>
+__device__ __forceinline__ int pm1_world_sum(const GT *g, int npad, unsigned long long w, int NP) {
+    int gs = 0;
+    for (int t0 = 0; t0 < NP; t0 += 32) {
+        const uint32_t b = (uint32_t)(w >> t0);
+        const int m = min(32, NP - t0);
+#pragma unroll 8
+        for (int t = 0; t < m; ++t) {
+            const int x = (int)g[(t0 + t) * npad];
+            gs += (b >> t) & 1u ? x : -x;
+        }
+    }
+    return gs;
+}
+
 // One warp sweeps slice t; one Philox call per lane serves four blocks.
 template <typename GT>
 __device__ __forceinline__ void pm1_sweep_slice(const uint32_t *Jw, uint32_t *S, GT *G, unsigned long long *Wc,
@@ -448,13 +465,7 @@ __global__ void __launch_bounds__(1024, 1) ring_pm1_kernel(RingParams p) {
             const OrdT *ord = feed_take(feed);
             for (int i = threadIdx.x; i < npad; i += blockDim.x) {
                 const int q = i >> 5;
-                int gs = 0;
-                if (i < n)
-                    for (int t = 0; t < NP; ++t) {
-                        const int g = (int)G[t * npad + i];
-                        gs += ((S[t * nw + q] >> lane) & 1u) ? g : -g;
-                    }
-                Gs[i] = gs;
+                Gs[i] = i < n ? pm1_world_sum(G + i, npad, Wc[i], NP) : 0;
                 if ((q & 3) == 0) {  // positions q*32 + lane .. + 96: one Philox call
                     const U4 r = philox((uint32_t)(((q >> 2) << 5) | lane), (uint32_t)slot, sigma, DOM_WORLD, R.key);
                     uw[i] = u24(r.x);
@@ -538,13 +549,7 @@ __global__ void __launch_bounds__(1024, 1) ring_pm1_kernel(RingParams p) {
             // holds one 32-spin block, so lane == spin & 31)
             for (int i = threadIdx.x; i < npad; i += blockDim.x) {
                 const int q = i >> 5;
-                int gs = 0;
-                if (i < n)
-                    for (int t = 0; t < NP; ++t) {
-                        const int g = (int)G[t * npad + i];
-                        gs += ((S[t * nw + q] >> lane) & 1u) ? g : -g;
-                    }
-                Gs[i] = gs;
+                Gs[i] = i < n ? pm1_world_sum(G + i, npad, Wc[i], NP) : 0;
                 if ((q & 3) == 0) {  // one Philox call per lane serves blocks q .. q+3 (npad: a multiple of 128)
                     const U4 r = philox((uint32_t)(((q >> 2) << 5) | lane), (uint32_t)slot, sigma, DOM_WORLD, R.key);
                     uw[i] = u24(r.x);
