@@ -784,7 +784,10 @@ static void (*slab_kernel(const RingPlan &pl))(RingParams) {
     return pl.ref_order ? ring_slab_kernel<uint32_t, true> : ring_slab_kernel<uint32_t, false>;
 }
 static void (*dense_kernel(const RingPlan &pl))(RingParams) {
-    return pl.ref_order ? ring_dense_kernel<true> : ring_dense_kernel<false>;
+    // how many columns of a flipped row a warp has in flight: dense_update_wide
+    if (dense_ld(pl.n_max) > 256)
+        return pl.ref_order ? ring_dense_kernel<true, true> : ring_dense_kernel<false, true>;
+    return pl.ref_order ? ring_dense_kernel<true, false> : ring_dense_kernel<false, false>;
 }
 
 // One launch of the planned ring kernel over steps [rp.step0, rp.step1).

@@ -28,7 +28,7 @@
 //   n = 24,  P = 32, 1 read,    50 steps of 20 + 5 sweeps   31.5 -> 12.0 ms
 //   n = 200, P = 32, 32 reads,  50 steps of 20 + 5 sweeps   85.3 -> 30.4 ms
 //   n = 200, P = 32, 600 reads, 20 steps of 20 + 5 sweeps  151.9 -> 67.5 ms
-//   n = 900, P = 16, 100 reads, 40 steps of 2 + 1 sweeps    76.6 -> 18.2 ms
+//   n = 900, P = 16, 100 reads, 40 steps of 2 + 1 sweeps    76.6 -> 14.7 ms
 // What is left is the chain of votes: at n = 24 each further slice adds 0.26 us
 // (500 cycles) to a sweep.  Not kept: the couplings of a block in a shared-memory
 // tile (its gather cost what it saved), J in shared memory (48.7 against
@@ -197,19 +197,44 @@ __device__ __forceinline__ void dense_update_cols(const float *J, int ld, float 
         if (col + 128 * c < ld) *reinterpret_cast<ulonglong2 *>(gt + col + 128 * c) = g[c];
 }
 
-__device__ __forceinline__ void dense_update(const float *J, int ld, float *gt, uint32_t F, int i, uint32_t ups,
-                                             int lane) {
-    __syncwarp();
+// More than 256 fields (WIDE): four groups at a time, so that 512 columns of a
+// row are in flight at once, in a function of its own (its registers would
+// push the block's state out).  Two groups at a time against this:
+//   n = 900,  P = 16, 100 reads, 40 steps of 2 + 1 sweeps  16.3 -> 14.7 ms
+//   n = 400,  P = 32, 40 reads,  20 steps of 20 + 5        29.1 -> 27.7 ms
+//   n = 280,  the same                                      20.8 -> 20.7 ms
+//   n = 1500, P = 16, 20 reads,  5 steps of 20 + 5          40.8 -> 33.0 ms
+// At most 256 fields keep the loop in line: the call costs there (n = 24
+// 10.9 -> 11.5 ms, n = 200 28.9 -> 31.5 ms), and both forms in one kernel spill.
+// Eight groups at a time spill too (n = 900 27.0 ms).
+__device__ __noinline__ void dense_update_wide(const float *J, int ld, float *gt, uint32_t F, int i, uint32_t ups,
+                                               int lane) {
     int base = 0;
+#pragma unroll 1
+    for (; base + 256 < ld; base += 512) dense_update_cols<4>(J, ld, gt, F, i, ups, base, lane);
 #pragma unroll 1
     for (; base + 128 < ld; base += 256) dense_update_cols<2>(J, ld, gt, F, i, ups, base, lane);
     if (base < ld) dense_update_cols<1>(J, ld, gt, F, i, ups, base, lane);
+}
+
+template <bool WIDE>
+__device__ __forceinline__ void dense_update(const float *J, int ld, float *gt, uint32_t F, int i, uint32_t ups,
+                                             int lane) {
+    __syncwarp();
+    if (WIDE) {
+        dense_update_wide(J, ld, gt, F, i, ups, lane);
+    } else {
+        int base = 0;
+#pragma unroll 1
+        for (; base + 128 < ld; base += 256) dense_update_cols<2>(J, ld, gt, F, i, ups, base, lane);
+        if (base < ld) dense_update_cols<1>(J, ld, gt, F, i, ups, base, lane);
+    }
     __syncwarp();
 }
 
 // One block of 32 positions of slice t (ORD: qanneal's order, spins ord[...];
 // else the checkerboard, spins ascending).
-template <bool ORD>
+template <bool ORD, bool WIDE>
 __device__ __forceinline__ int dense_block(const float *J, int ld, float *gt, unsigned long long *Wc, const float *h,
                                            const OrdT *ord, int n, int nw, int q, int t, int tp, int tn, uint32_t rw,
                                            float B, float T4, int lane, const SpinPipe &pp) {
@@ -297,13 +322,13 @@ __device__ __forceinline__ int dense_block(const float *J, int ld, float *gt, un
         __threadfence_block();
     }
     if ((F >> lane) & 1u) atomicXor(reinterpret_cast<uint32_t *>(Wc + i) + (t >> 5), 1u << (t & 31));
-    if (F) dense_update(J, ld, gt, F, i, ups, lane);
+    if (F) dense_update<WIDE>(J, ld, gt, F, i, ups, lane);
     return __popc(F);
 }
 
 // Slices t0, t0 + dt, ... < t1 of one slice sweep, one warp; the number of
 // flips.  cell: the ring's first RNG cell.
-template <bool ORD>
+template <bool ORD, bool WIDE>
 __device__ __noinline__ int dense_sweep(const float *J, uint32_t ord, unsigned long long *err, int n, int NP,
                                         int t0, int t1, int dt, float B, float T4, uint64_t key, uint32_t cell,
                                         uint32_t sigma, uint32_t tag) {
@@ -317,8 +342,9 @@ __device__ __noinline__ int dense_sweep(const float *J, uint32_t ord, unsigned l
 #pragma unroll 1
         for (int q = 0; q < nw; ++q) {
             if ((q & 3) == 0) r = philox((uint32_t)(((q >> 2) << 5) | lane), cell + (uint32_t)t, sigma, tag, key);
-            flips += dense_block<ORD>(J, ld, dsm<float>(L.G) + t * ld, dsm<unsigned long long>(L.W), dsm<float>(L.h),
-                                      dsm<OrdT>(ord), n, nw, q, t, tp, tn, pick(r, q & 3), B, T4, lane, pp);
+            flips += dense_block<ORD, WIDE>(J, ld, dsm<float>(L.G) + t * ld, dsm<unsigned long long>(L.W),
+                                            dsm<float>(L.h), dsm<OrdT>(ord), n, nw, q, t, tp, tn, pick(r, q & 3), B,
+                                            T4, lane, pp);
         }
     }
     return flips;
@@ -326,7 +352,7 @@ __device__ __noinline__ int dense_sweep(const float *J, uint32_t ord, unsigned l
 
 // One worldline sweep, whole CTA of W warps (ends with a barrier); the number
 // of moves accepted.
-template <bool ORD>
+template <bool ORD, bool WIDE>
 __device__ __noinline__ int dense_worldlines(const float *J, uint32_t ordo, int n, int NP, float B,
                                              uint64_t key, uint32_t slot, uint32_t sigma) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
@@ -408,7 +434,7 @@ __device__ __noinline__ int dense_worldlines(const float *J, uint32_t ordo, int 
         const int isp = dsm<int>(L.wsp)[lane];
         const unsigned long long wo = dsm<unsigned long long>(L.wold)[lane];
         for (int t = warp; t < NP; t += W)
-            dense_update(J, ld, G + t * ld, F, isp, __ballot_sync(FULL, ((wo >> t) & 1ull) != 0ull), lane);
+            dense_update<WIDE>(J, ld, G + t * ld, F, isp, __ballot_sync(FULL, ((wo >> t) & 1ull) != 0ull), lane);
         if (warp == 0 && ((F >> lane) & 1u)) Wc[isp] = wo ^ pmask;
         moves += __popc(F);
         __syncthreads();
@@ -419,7 +445,7 @@ __device__ __noinline__ int dense_worldlines(const float *J, uint32_t ordo, int 
 
 
 // ORD: qanneal's update order.
-template <bool ORD>
+template <bool ORD, bool WIDE>
 __global__ void __launch_bounds__(512, 1) ring_dense_kernel(RingParams p) {
     const RingDev R = p.rings[blockIdx.x];
     const ProbDev *Pd = p.probs + R.prob;
@@ -449,7 +475,8 @@ __global__ void __launch_bounds__(512, 1) ring_dense_kernel(RingParams p) {
 
     const unsigned long long pmask = NP == 64 ? ~0ull : ((1ull << NP) - 1ull);
     const int slot = p.slot ? p.slot[blockIdx.x] : R.k;
-    OrderFeed feed = feed_open(ORD ? dsm<OrdT>(L.ord0) : nullptr, ORD ? dsm<OrdT>(L.ord1) : nullptr, ORD ? p.ordg + blockIdx.x * p.ord_ring : nullptr, p.ord_stride, n,
+    OrderFeed feed = feed_open(ORD ? dsm<OrdT>(L.ord0) : nullptr, ORD ? dsm<OrdT>(L.ord1) : nullptr,
+                               ORD ? p.ordg + blockIdx.x * p.ord_ring : nullptr, p.ord_stride, n,
                                ORD ? (p.step1 - p.step0) * p.ord_per_step : 0);
     unsigned long long att_s = 0, acc_s = 0, att_w = 0, acc_w = 0;
     double bestE = p.best_E[blockIdx.x];
@@ -484,15 +511,15 @@ __global__ void __launch_bounds__(512, 1) ring_dense_kernel(RingParams p) {
                 ord = (uint32_t)(reinterpret_cast<const unsigned char *>(feed_take(feed)) - dense_sm);
             }
             if (ORD) {
-                acc_s += (unsigned long long)dense_sweep<true>(J, ord, p.counters + 4, n, NP, warp, NP, W, B, T4, R.key,
-                                                               (uint32_t)(slot * NP), sigma, tag);
+                acc_s += (unsigned long long)dense_sweep<true, WIDE>(J, ord, p.counters + 4, n, NP, warp, NP, W, B, T4,
+                                                                     R.key, (uint32_t)(slot * NP), sigma, tag);
                 __syncthreads();
             } else {
                 for (int ph = 0; ph < 3; ++ph) {
                     const int cnt = phase_count(NP, ph), b = phase_slice(NP, ph, 0);
-                    acc_s += (unsigned long long)dense_sweep<false>(J, 0, nullptr, n, NP, b + 2 * warp, b + 2 * cnt,
-                                                                    2 * W, B, T4, R.key, (uint32_t)(slot * NP), sigma,
-                                                                    tag);
+                    acc_s += (unsigned long long)dense_sweep<false, WIDE>(J, 0, nullptr, n, NP, b + 2 * warp,
+                                                                          b + 2 * cnt, 2 * W, B, T4, R.key,
+                                                                          (uint32_t)(slot * NP), sigma, tag);
                     if (cnt) __syncthreads();
                 }
             }
@@ -514,7 +541,7 @@ __global__ void __launch_bounds__(512, 1) ring_dense_kernel(RingParams p) {
             const uint32_t sigma = (uint32_t)(step * p.wls + sw);
             const uint32_t ord =
                 ORD ? (uint32_t)(reinterpret_cast<const unsigned char *>(feed_take(feed)) - dense_sm) : 0;
-            const int mv = dense_worldlines<ORD>(J, ord, n, NP, B, R.key, (uint32_t)slot, sigma);
+            const int mv = dense_worldlines<ORD, WIDE>(J, ord, n, NP, B, R.key, (uint32_t)slot, sigma);
             if (threadIdx.x == 0) {
                 att_w += (unsigned long long)n;
                 acc_w += (unsigned long long)mv;

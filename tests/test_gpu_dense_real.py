@@ -12,10 +12,12 @@ from test_gpu_parity_sa_sqa import oracle_model
 
 pytestmark = pytest.mark.gpu
 
-# block edges (31, 32, 33), row edges (n % 4, 128 and 256 columns), one slice,
-# two, a number that is no multiple of the warps, more than one slice a warp
+# block edges (31, 32, 33), row edges (n % 4, groups of 128 columns: two at a time
+# up to 256, four beyond), one slice, two, a number that is no multiple of
+# the warps, more than one slice a warp
 CASES = [(1, 4, 1, 1), (31, 1, 1, 0), (65, 1, 1, 2), (32, 2, 1, 1), (33, 3, 2, 1), (64, 16, 1, 2), (127, 17, 1, 1), (129, 5, 1, 1),
-         (257, 33, 1, 1), (130, 64, 1, 1), (514, 8, 1, 1)]
+         (257, 33, 1, 1), (130, 64, 1, 1), (514, 8, 1, 1),
+         (256, 3, 1, 1), (388, 4, 1, 1), (641, 3, 1, 1), (770, 2, 1, 1)]
 
 
 @pytest.mark.parametrize("order", ["reference", "checkerboard"])
