@@ -25,8 +25,8 @@
 // Spins live as worldline words (bit t of W[i]: slice t), P <= 64.
 //
 // Measured (solve() on a real QUBO, the whole call; before: ring_kernel):
-//   n = 24,  P = 32, 1 read,    50 steps of 20 + 5 sweeps   31.5 -> 12.0 ms
-//   n = 200, P = 32, 32 reads,  50 steps of 20 + 5 sweeps   85.3 -> 30.4 ms
+//   n = 24,  P = 32, 1 read,    50 steps of 20 + 5 sweeps   31.5 -> 10.9 ms
+//   n = 200, P = 32, 32 reads,  50 steps of 20 + 5 sweeps   85.3 -> 28.8 ms
 //   n = 200, P = 32, 600 reads, 20 steps of 20 + 5 sweeps  151.9 -> 67.5 ms
 //   n = 900, P = 16, 100 reads, 40 steps of 2 + 1 sweeps    76.6 -> 14.7 ms
 // What is left is the chain of votes: at n = 24 each further slice adds 0.26 us
@@ -44,8 +44,8 @@ namespace qa {
 __host__ __device__ inline int dense_ld(int n) { return (n + 3) & ~3; }
 
 // Shared memory of one ring: byte offsets.  The sweeps are functions of their
-// own (a slice sweep and the rest of the kernel together would not fit the 64
-// registers of a 1024-thread CTA) and take offsets, so that their accesses
+// own (a slice sweep and the rest of the kernel together would not fit the 128
+// registers of a 512-thread CTA) and take offsets, so that their accesses
 // stay shared-memory ones.
 struct DenseLay {
     uint32_t G, W, h, uw, cellE, gb, wold, wsp, mask, part, flag, ord0, ord1, prog, pbits, abortf, total;
@@ -165,9 +165,8 @@ __device__ __forceinline__ unsigned long long pack2(float c) {
 }
 
 // Fields of one slice after the spins of lanes F flipped (lane's spin i, old
-// bits ups by lane): NC groups of 128 fields from column base on.  Two flips
-// at a time, so that the loads of eight rows' pieces are in flight; an odd
-// last one is paired with itself at weight 0 (couplings are finite here).
+// bits ups by lane): NC groups of 128 fields from column base on, a flip's
+// pieces of its row in flight at once.
 template <int NC>
 __device__ __forceinline__ void dense_update_cols(const float *J, int ld, float *gt, uint32_t F, int i, uint32_t ups,
                                                   int base, int lane) {
