@@ -320,7 +320,7 @@ template <class WT, bool ORD>
 __global__ void __launch_bounds__(256, 3) ring_slab_kernel(RingParams p) {
     const RingDev R = p.rings[blockIdx.x];
     const ProbDev *Pd = p.probs + R.prob;
-    const int NP = p.P, W = p.W, n = Pd->n, nw = Pd->nw, n32 = nw * 32, nsb = (n + 127) >> 7;
+    const int NP = p.P, W = p.W, n = Pd->n, nw = Pd->nw, nsb = (n + 127) >> 7;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint4 *slab = Pd->spslab;
     const float *h32 = Pd->h32;
