@@ -127,7 +127,9 @@ __global__ void __launch_bounds__(32 * kSaWarps) sa_dense_kernel(SAParams p) {
     long long x = 0;
     for (int step = 0; step < p.steps; ++step) {
         const float B = p.B[step], eB = eps / B;
-        const bool plain = B > 1e-30f && B < 1e30f;  // else every block takes the exact test
+        // else every lane takes the exact test: no s g is below -inf or reaches a NaN
+        // (an upper limit of +inf would accept an infinite field at B = 0)
+        const bool plain = B > 1e-30f && B < 1e30f;
         for (int sw = 0; sw < p.spb; ++sw, ++x) {
             if (warp != 0) {
                 if (x + 1 < sweeps) draw(x + 1, warp - 1, ((int)blockDim.x >> 5) - 1);
@@ -140,7 +142,7 @@ __global__ void __launch_bounds__(32 * kSaWarps) sa_dense_kernel(SAParams p) {
                     const float hi = h[i], gf = (float)G[i], sh = sbit ? hi : -hi;
                     float sg = sbit ? gf : -gf;
                     const float th = c[i] - sh, e = __fmaf_rn(1e-6f, fabsf(c[i]) + fabsf(sh), eB);
-                    const float lo = plain ? th - e : -f_inf(), up = plain ? th + e : f_inf();
+                    const float lo = plain ? th - e : -f_inf(), up = plain ? th + e : __int_as_float(0x7fffffff);
                     uint32_t pend = n - (q << 5) >= 32 ? FULL : (1u << (n - (q << 5))) - 1u;
                     uint32_t m = __ballot_sync(FULL, sg >= lo) & pend;
                     if (!m) continue;
