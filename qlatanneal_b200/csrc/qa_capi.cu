@@ -1833,6 +1833,19 @@ static int sa_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_problem
     bool real = kind == K_DENSE && !traces && !pm1 && sa_dense_smem_bytes<false>(n_max) <= (size_t)ctx->smem_optin &&
                 !std::getenv("QA_DISABLE_DENSE");
     for (int p = 0; p < n_problems && real; ++p) real = problems[p]->plain_j;
+    auto sa_kern = pm1 ? sa_dense_kernel<true> : sa_dense_kernel<false>;
+    const size_t sa_smem = pm1 ? sa_dense_smem_bytes<true>(n_max) : sa_dense_smem_bytes<false>(n_max);
+    int sa_w = sa_warps(n_max);
+    if (pm1 || real) {
+        QA_TRY(opt_in_smem(ctx, (const void *)sa_kern, sa_smem));
+        if (nr > ctx->sms) {
+            int many = 0, one = 0;  // CTAs an SM
+            QA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&many, sa_kern, 32 * sa_w, sa_smem));
+            QA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, sa_kern, 32, sa_smem));
+            sa_w = sa_form(pm1, n_max, nr, (long long)many * ctx->sms, (long long)one * ctx->sms);
+            real = real && sa_w > 0;
+        }
+    }
     QA_CK(cudaEventRecord(ctx->ev[0], ctx->stream));
     QA_TRY(init_state(ctx, kind, d_probs, d_rings, nr, d_spins, d_fields, 1, n_max, L.nw_max, DOM_INIT, !pm1));
     const int nwp = (L.nw_max + 3) & ~3, np4 = (n_max + 3) & ~3;
@@ -1848,10 +1861,7 @@ static int sa_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_problem
     QA_CK(cudaEventRecord(ctx->ev[1], ctx->stream));
     int rc = QA_OK;
     if (pm1 || real) {
-        auto kern = pm1 ? sa_dense_kernel<true> : sa_dense_kernel<false>;
-        const size_t sm1 = pm1 ? sa_dense_smem_bytes<true>(n_max) : sa_dense_smem_bytes<false>(n_max);
-        QA_TRY(opt_in_smem(ctx, (const void *)kern, sm1));
-        kern<<<nr, 32 * sa_warps(n_max), sm1, ctx->stream>>>(sp);
+        sa_kern<<<nr, 32 * sa_w, sa_smem, ctx->stream>>>(sp);
         QA_CK(cudaGetLastError());
     } else {
         dispatch_kind(kind, [&](auto K) {

@@ -6,8 +6,9 @@
 // chain, and a warp alone on its SM issues an instruction about every four
 // cycles, so the time is what the chain's warp has to do:
 //  * up to three warps draw the next sweep's uniforms and turn them into limits
-//    on s(h + g) while the first sweeps: rejecting a block of 32 spins is a few
-//    loads, a handful of operations and one vote;
+//    on s(h + g) while the first sweeps (sa_form; with many reads the first draws
+//    them itself): rejecting a block of 32 spins is a few loads, a handful of
+//    operations and one vote;
 //  * a block with flips is resolved on registers against the limits (exact test
 //    in between).  +-1 couplings (PM1): the block's flips change the fields of
 //    all spins at once, from bits in shared memory.  Others: a flip's float32
@@ -31,6 +32,23 @@ namespace qa {
 constexpr int kSaWarps = 4;
 // The sweeping warp and one for each 128 uniforms of a sweep, up to three.
 static inline int sa_warps(int n) { return 1 + std::min(kSaWarps - 1, (n + 127) / 128); }
+
+// How nr reads run: warps a read, 0 for sa_kernel.  many / one: reads resident on
+// the GPU at once with sa_warps(n) warps and with one (which draws its own limits).
+// Drawing ahead shortens a lone chain by up to 15% and costs residency (real
+// couplings, n = 256: 592 reads against 1776), so it stops where the reads no longer
+// fit, with two warps at half of that, where the SMs are busy without it (+-1,
+// n = 64, 600 reads: 0.46 ms either way, 1000 reads 0.52 -> 0.48).  Real, n = 1000,
+// 1000 reads 13.2 -> 5.0 ms; n = 256, 4000 reads 11.5 -> 5.6; +-1, n = 64, 8000 reads
+// 2.72 -> 1.60.  +-1 from n = 400 on is bounded by shared memory either way (2%
+// slower with one warp).  Reads beyond that of small real models go to sa_kernel,
+// whose 64 registers hold 32 reads an SM against 12 here (n = 64, 4000 reads: one
+// warp 2.00, sa_kernel 1.62 ms; n = 128, 4700 reads: 3.93 and 4.42).
+static inline int sa_form(bool pm1, int n, long long nr, long long many, long long one) {
+    if (nr <= (sa_warps(n) > 2 ? many : many / 2)) return sa_warps(n);
+    if (!pm1 && n < 96 && nr > one) return 0;
+    return one > many ? 1 : sa_warps(n);
+}
 
 template <bool PM1>
 __host__ __device__ inline size_t sa_dense_smem_bytes(int n) {
@@ -134,6 +152,10 @@ __global__ void __launch_bounds__(32 * kSaWarps) sa_dense_kernel(SAParams p) {
             if (warp != 0) {
                 if (x + 1 < sweeps) draw(x + 1, warp - 1, ((int)blockDim.x >> 5) - 1);
             } else {
+                if (blockDim.x == 32 && x > 0) {  // nobody drew ahead
+                    draw(x, 0, 1);
+                    __syncwarp();
+                }
                 const float *c = cb + (x & 1) * npad;
 #pragma unroll 1
                 for (int q = 0; q < nw; ++q) {

@@ -1,0 +1,43 @@
+"""A call that a special kernel takes is not slower than the general path it took
+before (the switch in the second column brings that back).  Where the rules of
+the dispatch put the line wrong the special path took 1.3 to 6 times as long;
+the bound is 1.25 on the fastest of six runs of each side, taken in turn.
+"""
+import numpy as np
+import pytest
+
+import qlatanneal_b200 as qa
+from qlatanneal_b200.instances import dense_real
+
+pytestmark = pytest.mark.gpu
+
+
+def sa_real(n, reads):
+    """Chains in flight, not the time of one chain, bound many reads."""
+    betas = np.geomspace(0.3, 3.0, 20) * 1.7 / np.sqrt(n)
+    ann = qa.Annealer(qa.DenseIsing(*dense_real(n, 1)), qa.AnnealSchedule.from_betas(betas))
+    return ann, lambda: ann.run_reads(5, reads=reads, seed=1)
+
+
+SHAPES = [
+    (sa_real, "QA_DISABLE_DENSE", (24, 4000)),
+    (sa_real, "QA_DISABLE_DENSE", (64, 2000)),
+    (sa_real, "QA_DISABLE_DENSE", (256, 4000)),
+]
+
+
+@pytest.mark.parametrize("make,switch,shape", SHAPES, ids=lambda v: getattr(v, "__name__", None))
+def test_not_slower_than_the_general_path(monkeypatch, make, switch, shape):
+    ann, call = make(*shape)
+    special, general = [], []
+    try:
+        for _ in range(7):
+            call()
+            special.append(ann.last_stats.sweep_ms)
+            monkeypatch.setenv(switch, "1")
+            call()
+            general.append(ann.last_stats.sweep_ms)
+            monkeypatch.delenv(switch)
+    finally:
+        qa.set_update_order("reference")
+    assert min(special[1:]) <= 1.25 * min(general[1:])
