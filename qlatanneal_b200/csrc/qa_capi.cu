@@ -716,6 +716,8 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
     // sparse rows in neighbour records: spins outside, slices inside
     pl->slab = !clusters && kind == K_SPARSE && P <= 64 && !std::getenv("QA_DISABLE_SPARSE_INT") &&
                !std::getenv("QA_DISABLE_SLAB") && slab_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin;
+    pl->slab = pl->slab && (slab_pays(P, n_max, n_rings, ctx->sms, ref_order) ||
+                            sparse_smem_bytes(P, n_max, ref_order) > (size_t)ctx->smem_optin);
     for (int p = 0; p < np && pl->slab; ++p) pl->slab = probs[p]->dev.spslab != nullptr;
     if (pl->slab) {
         pl->wide = P > 32;

@@ -32,6 +32,9 @@
 // ring's warps then follow four steps behind each other: 55 to 83 ms), sleeping
 // in the waits (no change).
 #pragma once
+#include <algorithm>
+#include <cmath>
+
 #include "qa_dense.cuh"
 #include "qa_sparse.cuh"
 
@@ -65,6 +68,23 @@ __host__ __device__ inline SlabLay slab_layout(int P, int n, int wbytes, bool re
 }
 __host__ __device__ inline size_t slab_smem_bytes(int P, int n, bool ref_order) {
     return slab_layout(P, n, P <= 32 ? 4 : 8, ref_order).total;
+}
+
+// Whether a call's rings run here or on ring_sparse_kernel.  A sweep is P slices one
+// after another for each 128 spins, so in the checkerboard order, where
+// ring_sparse_kernel sweeps P / 2 slices side by side, few spins and many slices are
+// faster there.  In units of one slice here (58 us of 50 sweeps) a sweep costs P;
+// there (n + 20) / 7.5, times what the rings share an SM's 32 such warps.  P = 32, one
+// ring, 50 slice sweeps: n = 40 0.64 / 1.74 ms there / here, n = 128 1.34 / 2.02,
+// n = 256 2.27 / 1.92; P = 16: n = 64 0.75 / 0.94, n = 128 1.20 / 1.01; P = 64, n = 40:
+// 148 rings 0.90 / 3.86, 600 rings 4.7 / 4.1.  In qanneal's order only one slice of one
+// block is faster there (n = 16, P = 1, one ring: 0.124 / 0.160 ms).
+inline bool slab_pays(int P, int n, int rings, int sms, bool ref_order) {
+    if (ref_order) return P > 1 || n > 32;
+    const int w = (P + 1) / 2, per_sm = std::max(1, 32 / w);
+    const double share = 1.0 + 1.5 * std::max(0.0, (double)rings / sms - 1.0) * w / 32.0;
+    const double waves = std::ceil((double)rings / ((double)per_sm * sms));
+    return (n + 20) * std::max(share, waves) > 7.5 * P;
 }
 
 __device__ __forceinline__ int popc_of(uint32_t w) { return __popc(w); }

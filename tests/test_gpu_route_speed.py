@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import qlatanneal_b200 as qa
-from qlatanneal_b200.instances import dense_real
+from qlatanneal_b200.instances import dense_real, regular3
 
 pytestmark = pytest.mark.gpu
 
@@ -19,10 +19,23 @@ def sa_real(n, reads):
     return ann, lambda: ann.run_reads(5, reads=reads, seed=1)
 
 
+def sparse_checkerboard(n, P, reads):
+    """Few spins, many slices, slices side by side."""
+    qa.set_update_order("checkerboard")
+    ann = qa.SQAAnnealer(qa.SparseIsing(*regular3(n, 1), n),
+                         qa.SQASchedule.from_vectors(P * np.linspace(0.1, 2.0, 10), np.linspace(2.0, 0.05, 10)), P)
+    return ann, lambda: ann.run_reads(5, 1, reads=reads, seed=1)
+
+
 SHAPES = [
     (sa_real, "QA_DISABLE_DENSE", (24, 4000)),
     (sa_real, "QA_DISABLE_DENSE", (64, 2000)),
     (sa_real, "QA_DISABLE_DENSE", (256, 4000)),
+    (sparse_checkerboard, "QA_DISABLE_SLAB", (40, 32, 1)),
+    (sparse_checkerboard, "QA_DISABLE_SLAB", (40, 64, 200)),
+    (sparse_checkerboard, "QA_DISABLE_SLAB", (128, 64, 32)),
+    (sparse_checkerboard, "QA_DISABLE_SLAB", (512, 32, 32)),
+    (sparse_checkerboard, "QA_DISABLE_SLAB", (128, 16, 600)),
 ]
 
 
