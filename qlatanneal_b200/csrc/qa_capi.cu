@@ -740,14 +740,11 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
     pl->dense = !clusters && kind == K_DENSE && P <= 64 && !std::getenv("QA_DISABLE_DENSE") &&
                 dense_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin;
     for (int p = 0; p < np && pl->dense; ++p) pl->dense = probs[p]->plain_j;
+    const int dense_w = dense_warps(P, n_max, n_rings, ctx->sms, ref_order);
+    pl->dense = pl->dense && dense_w > 0;
     if (pl->dense) {
         pl->smem = dense_smem_bytes(P, n_max, ref_order);
-        // one warp per slice up to 16 (the kernel's 128 registers a thread);
-        // 8 where the rings are at least two waves and blocks are few (n <= 256):
-        // two rings on an SM then beat one with twice the warps (P = 32,
-        // 600 rings: n = 24 23.3 -> 17.7 ms, n = 64 36.8 -> 28.3, n = 200
-        // 69.9 -> 66.4; 300 rings of n = 900 25.1 -> 28.2, so not there)
-        if (ctx->tune.warps_per_ring <= 0) pl->W = std::min(P, n_rings >= 2 * ctx->sms && n_max <= 256 ? 8 : 16);
+        if (ctx->tune.warps_per_ring <= 0) pl->W = dense_w;
         pl->W = std::min(pl->W, 16);
         return QA_OK;
     }

@@ -36,6 +36,8 @@
 // 30 -> 48 ms), a shorter loop for blocks whose predecessor is done (the
 // chain, not the instruction count, is the time).
 #pragma once
+#include <algorithm>
+
 #include "qa_pm1.cuh"
 
 namespace qa {
@@ -82,6 +84,24 @@ __host__ __device__ inline DenseLay dense_layout(int P, int n, bool ref_order) {
 }
 __host__ __device__ inline size_t dense_smem_bytes(int P, int n, bool ref_order) {
     return dense_layout(P, n, ref_order).total;
+}
+
+// Warps of a ring, 0 for ring_kernel.  One per slice up to 16 (128 registers a
+// thread); 8 where the rings are at least two waves and blocks are few (n <= 256):
+// two rings on an SM then beat one with twice the warps (P = 32, 600 rings: n = 24
+// 23.3 -> 17.7 ms, n = 64 36.8 -> 28.3, n = 200 69.9 -> 66.4; 300 rings of n = 900
+// 25.1 -> 28.2, so not there).  In the checkerboard order half the slices rest: with
+// more rings than SMs no more warps than slices of a phase (18 slice sweeps, P = 8:
+// n = 200, 1000 rings 1.47 -> 0.92 ms; n = 24, 450 rings 0.195 -> 0.119), and with at
+// most two blocks nothing is left of the shorter chain where those no longer fit on the
+// SMs, 16 warps each: ring_kernel has 64 registers (n = 24: P = 8, 3000 rings 0.56 here
+// with 4 warps / 0.46 there; P = 24, 300 rings 0.35 / 0.29).
+inline int dense_warps(int P, int n, int rings, int sms, bool ref_order) {
+    const int w = std::min(P, rings >= 2 * sms && n <= 256 ? 8 : 16);
+    if (ref_order && P > 1) return w;
+    const int phase = (P + 1) / 2;
+    if (n <= 64 && rings > sms * (16 / phase)) return 0;
+    return rings > sms ? std::min(w, phase) : w;
 }
 
 extern __shared__ __align__(16) unsigned char dense_sm[];

@@ -27,6 +27,14 @@ def sparse_checkerboard(n, P, reads):
     return ann, lambda: ann.run_reads(5, 1, reads=reads, seed=1)
 
 
+def dense_checkerboard(n, P, reads):
+    """Many rings: the slices of a phase at work on all SMs, not the chain of one."""
+    qa.set_update_order("checkerboard")
+    ann = qa.SQAAnnealer(qa.DenseIsing(*dense_real(n, 1)), qa.SQASchedule.from_vectors(
+        P * np.linspace(0.1, 3.0, 6) / np.sqrt(n), np.linspace(2.0, 0.05, 6)), P)
+    return ann, lambda: ann.run_reads(3, 0, reads=reads, seed=1)
+
+
 SHAPES = [
     (sa_real, "QA_DISABLE_DENSE", (24, 4000)),
     (sa_real, "QA_DISABLE_DENSE", (64, 2000)),
@@ -36,6 +44,10 @@ SHAPES = [
     (sparse_checkerboard, "QA_DISABLE_SLAB", (128, 64, 32)),
     (sparse_checkerboard, "QA_DISABLE_SLAB", (512, 32, 32)),
     (sparse_checkerboard, "QA_DISABLE_SLAB", (128, 16, 600)),
+    (dense_checkerboard, "QA_DISABLE_DENSE", (12, 8, 3000)),
+    (dense_checkerboard, "QA_DISABLE_DENSE", (24, 12, 600)),
+    (dense_checkerboard, "QA_DISABLE_DENSE", (64, 5, 1000)),
+    (dense_checkerboard, "QA_DISABLE_DENSE", (200, 8, 600)),
 ]
 
 
