@@ -1601,13 +1601,16 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
     // flip updates grouped by target (terms of degree <= 4 only)
     bool small_terms = true;
     for (int t = 0; t < n_terms && small_terms; ++t) small_terms = tptr[t + 1] - tptr[t] <= 4;
-    std::vector<int> hub_ptr;
+    std::vector<uint4> hub_spin;
+    std::vector<uint32_t> hub_off;
     std::vector<int4> hub_rec;
     if (small_terms) {
-        hub_ptr.assign(n + 1, 0);
-        std::vector<std::vector<int4>> layer;  // layer k: the k-th record of each target
+        hub_spin.assign(n, make_uint4(0u, 0u, 0u, 0u));
+        hub_off.assign(1, 0u);
         struct U { int v, t, w1, w2; };
         std::vector<U> u;
+        std::vector<std::pair<int, int>> runs;  // the records of each target: (first, number)
+        std::vector<uint32_t> chunk_of(n, 0u);  // the last chunk (counted from 1) with the target
         for (int j = 0; j < n; ++j) {
             u.clear();
             for (int q = incptr[j]; q < incptr[j + 1]; ++q) {
@@ -1621,21 +1624,41 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
                     u.push_back({v, t, w[0], w[1]});
                 }
             }
+            if (u.empty()) continue;
             std::stable_sort(u.begin(), u.end(), [](const U &a, const U &b) { return a.v != b.v ? a.v < b.v : a.t < b.t; });
-            layer.clear();
-            for (size_t k = 0, l = 0; k < u.size(); ++k) {
-                l = k > 0 && u[k].v == u[k - 1].v ? l + 1 : 0;
-                if (layer.size() <= l) layer.emplace_back();
-                const float two = 2.0f * c32[u[k].t];
-                int bits;
-                std::memcpy(&bits, &two, 4);
-                layer[l].push_back(make_int4(u[k].v, u[k].w1, u[k].w2, bits));
+            runs.clear();
+            for (size_t k = 0; k < u.size(); ++k) {
+                if (k == 0 || u[k].v != u[k - 1].v) runs.push_back({(int)k, 0});
+                ++runs.back().second;
             }
-            for (auto &l : layer) {
-                l.resize((l.size() + 31) / 32 * 32, make_int4(-1, -1, -1, 0));
-                hub_rec.insert(hub_rec.end(), l.begin(), l.end());
+            // the first record of every target, then the second, ..; targets with the
+            // most records first, so that a chunk can run on into the next round
+            std::stable_sort(runs.begin(), runs.end(), [](const auto &a, const auto &b) { return a.second > b.second; });
+            const uint32_t c0 = (uint32_t)hub_off.size();  // this spin's first chunk, counted from 1
+            uint32_t in_chunk = 0;
+            size_t left = runs.size();
+            for (int round = 0; left > 0; ++round) {
+                while (left > 0 && runs[left - 1].second <= round) --left;
+                for (size_t r = 0; r < left; ++r) {
+                    const U &x = u[(size_t)(runs[r].first + round)];
+                    if (in_chunk == 32 || chunk_of[x.v] == (uint32_t)hub_off.size()) {
+                        hub_off.push_back((uint32_t)hub_rec.size());
+                        in_chunk = 0;
+                    }
+                    chunk_of[x.v] = (uint32_t)hub_off.size();
+                    const float two = 2.0f * c32[x.t];
+                    int bits;
+                    std::memcpy(&bits, &two, 4);
+                    hub_rec.push_back(make_int4(x.v, x.w1, x.w2, bits));
+                    ++in_chunk;
+                }
             }
-            hub_ptr[j + 1] = (int)(hub_rec.size() / 32);
+            hub_off.push_back((uint32_t)hub_rec.size());
+            const uint32_t chunks = (uint32_t)hub_off.size() - c0;
+            uint32_t sizes = 0;
+            for (uint32_t k = 0; k < std::min(4u, chunks); ++k)
+                sizes |= (hub_off[c0 + k] - hub_off[c0 + k - 1]) << (8 * k);
+            hub_spin[j] = make_uint4(hub_off[c0 - 1], sizes, c0 + 3, std::max(c0 + 3, c0 + chunks - 1));
         }
     }
     qa_problem *P = new qa_problem();
@@ -1653,7 +1676,8 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
     if (rc == QA_OK) rc = upload(P, c32.data(), c32.size(), &P->dev.coef32);
     if (rc == QA_OK) rc = upload(P, coeff, (size_t)n_terms, &P->dev.coef64);
     if (rc == QA_OK && small_terms) {
-        rc = upload(P, hub_ptr.data(), hub_ptr.size(), &P->dev.hub_ptr);
+        rc = upload(P, hub_spin.data(), hub_spin.size(), &P->dev.hub_spin);
+        if (rc == QA_OK) rc = upload(P, hub_off.data(), hub_off.size(), &P->dev.hub_off);
         if (rc == QA_OK) rc = upload(P, hub_rec.data(), hub_rec.size(), &P->dev.hub_rec);
         // one 16-byte record per term for the per-step energy scan
         std::vector<int4> trec(std::max(n_terms, 1), make_int4(-1, -1, -1, -1));

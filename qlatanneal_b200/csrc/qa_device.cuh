@@ -151,12 +151,14 @@ struct ProbDev {
     // bits J[m][32q .. 32q+31] (1 = +1; diagonal and padding bits 0); else null
     const uint32_t *Jw;
     // hubo with every term of degree <= 4: the field updates of a flip of
-    // spin j in chunks hub_ptr[j] .. hub_ptr[j+1] of 32 records (one load of a
-    // warp), hub_rec[32 c + lane] = {v, w1, w2, bits(2 J_t)}: target v (-1: no
-    // record), w1, w2 the term's other spins (-1: none).  A chunk holds a target
-    // once; a target's terms stand in increasing order, one chunk after another.
-    // Else null.
-    const int *hub_ptr;
+    // spin j in chunks of up to 32 records (one load of a warp), chunk c =
+    // hub_rec[hub_off[c] .. hub_off[c+1]).  Record {v, w1, w2, bits(2 J_t)}: target
+    // v, w1, w2 the term's other spins (-1: none).  A chunk holds a target once; a
+    // target's terms stand in increasing order, one chunk after another.
+    // hub_spin[j] = {first record, the sizes of the first four chunks in a byte each,
+    // first and end of the chunks after those}.  Else null.
+    const uint4 *hub_spin;
+    const uint32_t *hub_off;
     const int4 *hub_rec;
     // hubo with every term of degree <= 4: term t's spins {v0, v1, v2, v3}
     // (-1: none) in one 16-byte record, for the per-step energy scan; else null
@@ -171,6 +173,47 @@ struct ProbDev {
 };
 
 __device__ __forceinline__ int spin_of(const uint32_t *S, int i) { return ((S[i >> 5] >> (i & 31)) & 1u) ? 1 : -1; }
+
+// f on this lane's record (x < 0: none) of each chunk after the first of a spin with
+// hub_spin entry hs (the same in all lanes), in order, the warp in step before each; up
+// to four chunks' loads in flight.
+template <class F>
+__device__ __forceinline__ void hub_chunks(const uint4 &hs, const uint32_t *off, const int4 *rec, int lane, F f) {
+    const uint32_t size = hs.y >> 8;
+    if (size == 0u) return;
+    const int4 none = make_int4(-1, -1, -1, 0);
+    int4 r[4];
+    uint32_t at = hs.x + (hs.y & 255u);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t c = (size >> (8 * k)) & 255u;
+        r[k] = (uint32_t)lane < c ? __ldg(rec + at + lane) : none;
+        at += c;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        if ((size >> (8 * k)) & 255u) {
+            __syncwarp();
+            f(r[k]);
+        }
+#pragma unroll 1
+    for (uint32_t c = hs.z; c < hs.w; c += 4) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            r[k] = none;
+            if (c + k < hs.w) {
+                const uint32_t a = __ldg(off + c + k) + (uint32_t)lane;
+                if (a < __ldg(off + c + k + 1)) r[k] = __ldg(rec + a);
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+            if (c + k < hs.w) {
+                __syncwarp();
+                f(r[k]);
+            }
+    }
+}
 
 // Field update after spin j (old value so) flipped in one slice whose spin bits
 // (already holding the new value) are S and whose fields are g.  Whole warp
@@ -194,18 +237,17 @@ __device__ __forceinline__ void apply_flip(const ProbDev &P, float *g, const uin
         // one lane per target spin v, its terms in order: the same float
         // additions, in the same order per field, as the term-by-term loop
         const int sj = spin_of(S, j);  // S holds the new spin
-        const int a = __ldg(P.hub_ptr + j), b = __ldg(P.hub_ptr + j + 1);
-        for (int c = a; c < b; ++c) {
-            const int4 rc = __ldg(P.hub_rec + 32 * c + lane);
-            if (c > a) __syncwarp();
-            if (rc.x >= 0) {
-                int pr = sj;
-                if (rc.y >= 0) pr *= spin_of(S, rc.y);
-                if (rc.z >= 0) pr *= spin_of(S, rc.z);
-                const float two = __int_as_float(rc.w);
-                g[rc.x] = __fadd_rn(g[rc.x], pr > 0 ? two : -two);
-            }
-        }
+        const uint4 hs = __ldg(P.hub_spin + j);
+        auto add = [&](const int4 &rc) {
+            if (rc.x < 0) return;
+            int pr = sj;
+            if (rc.y >= 0) pr *= spin_of(S, rc.y);
+            if (rc.z >= 0) pr *= spin_of(S, rc.z);
+            const float two = __int_as_float(rc.w);
+            g[rc.x] = __fadd_rn(g[rc.x], pr > 0 ? two : -two);
+        };
+        if ((uint32_t)lane < (hs.y & 255u)) add(__ldg(P.hub_rec + hs.x + lane));
+        hub_chunks(hs, P.hub_off, P.hub_rec, lane, add);
     } else {
         const int q0 = __ldg(P.incptr + j), q1 = __ldg(P.incptr + j + 1);
         for (int q = q0; q < q1; ++q) {

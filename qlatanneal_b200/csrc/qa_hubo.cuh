@@ -3,8 +3,9 @@
 //
 // Same replay semantics as ring_kernel<K_HUBO>.  What bounds this path is the
 // chain of an accepted flip: its field updates, and the decisions after it.
-//  * a flip's updates are 32-record chunks (ProbDev::hub_rec), one coalesced load
-//    for the warp, asked for while the flip before is applied;
+//  * a flip's updates are chunks of up to 32 records (ProbDev::hub_rec), one
+//    coalesced load for the warp, the first asked for while the flip before is
+//    applied;
 //  * after a flip only lanes whose field it changed decide again (the inverse
 //    order tells which of the updated spins sit in the block);
 //  * worldline moves: a warp evaluates a block of 32 positions, the moves before
@@ -58,6 +59,22 @@ __host__ __device__ inline size_t hubo_smem_bytes(int P, int n, bool ref_order) 
     return hubo_layout(P, n, ref_order).total;
 }
 
+// The field updates of a flip (ProbDev::hub_spin, hub_off, hub_rec).
+struct HubRows {
+    const uint4 *spin;
+    const uint32_t *off;
+    const int4 *rec;
+};
+
+// Lane j's entry in all lanes, and this lane's record of its first chunk.
+__device__ __forceinline__ uint4 hub_of(const uint4 &hs, int j) {
+    return make_uint4(__shfl_sync(FULL, hs.x, j), __shfl_sync(FULL, hs.y, j), __shfl_sync(FULL, hs.z, j),
+                      __shfl_sync(FULL, hs.w, j));
+}
+__device__ __forceinline__ int4 hub_first(const HubRows &hr, uint32_t at, uint32_t sizes, int lane) {
+    return (uint32_t)lane < (sizes & 255u) ? __ldg(hr.rec + at + lane) : make_int4(-1, -1, -1, 0);
+}
+
 // One record's update after a flip of its spin (new value sj = +-1): S holds the
 // flip.
 __device__ __forceinline__ void hubo_add(const int4 &r, float *g, const uint32_t *S, int sj) {
@@ -79,7 +96,7 @@ __device__ __forceinline__ uint32_t hubo_touch(const int4 &r, const OrdT *inv, i
 
 // Slices t0, t0 + dt, .. < t1 of one slice sweep, one warp; the number of flips.
 template <bool ORD>
-__device__ __noinline__ int hubo_sweep(const int *hptr, const int4 *hrec, uint32_t ordo, unsigned long long *err, int n,
+__device__ __noinline__ int hubo_sweep(const HubRows hr, uint32_t ordo, unsigned long long *err, int n,
                                        int NP, int t0, int t1, int dt, float B, float T4, uint64_t key, uint32_t cell,
                                        uint32_t sigma, uint32_t tag) {
     const int lane = threadIdx.x & 31, nw = (n + 31) >> 5, ld = dense_ld(n);
@@ -102,7 +119,7 @@ __device__ __noinline__ int hubo_sweep(const int *hptr, const int4 *hrec, uint32
             const int pos = (q << 5) | lane;
             const bool valid = pos < n;
             const int i = valid ? (ORD ? (int)ord[pos] : pos) : 0;
-            const int c0 = __ldg(hptr + i), c1 = __ldg(hptr + i + 1);  // the spin's chunks
+            const uint4 hs = __ldg(hr.spin + i);  // the spin's chunks
             const float u = u24(pick(r, q & 3)), hi = h[i];
             const uint32_t sb = (St[i >> 5] >> (i & 31)) & 1u;
             const float Bs = sb ? B : -B, lim0 = accept_limit(u);
@@ -121,15 +138,15 @@ __device__ __noinline__ int hubo_sweep(const int *hptr, const int4 *hrec, uint32
             };
             uint32_t m = decide();
             if (m) {
-                auto chunk = [&](int j) {  // the first chunk of lane j's spin (nothing when it has none)
-                    const int a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
-                    return a < b ? __ldg(hrec + 32 * a + lane) : make_int4(-1, -1, -1, 0);
+                auto chunk = [&](int j) {
+                    return hub_first(hr, __shfl_sync(FULL, hs.x, j), __shfl_sync(FULL, hs.y, j), lane);
                 };
                 int j = __ffs(m) - 1;
                 int4 rec = chunk(j);
                 while (true) {
                     const uint32_t pend = j == 31 ? 0u : ~((2u << j) - 1u);
-                    const int jj = __shfl_sync(FULL, i, j), a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
+                    const int jj = __shfl_sync(FULL, i, j);
+                    const uint4 hj = hub_of(hs, j);
                     const int sj = __shfl_sync(FULL, sb, j) ? -1 : 1;  // the new spin
                     if (lane == 0) St[jj >> 5] ^= 1u << (jj & 31);
                     ++flips;
@@ -138,12 +155,11 @@ __device__ __noinline__ int hubo_sweep(const int *hptr, const int4 *hrec, uint32
                     __syncwarp();
                     hubo_add(rec, gt, St, sj);
                     uint32_t touch = hubo_touch<ORD>(rec, inv, q);
-                    for (int c = a + 1; c < b; ++c) {  // (chunks in order: a target's terms stay in order)
-                        const int4 x = __ldg(hrec + 32 * c + lane);
-                        __syncwarp();
+                    // (chunks in order: a target's terms stay in order)
+                    hub_chunks(hj, hr.off, hr.rec, lane, [&](const int4 &x) {
                         hubo_add(x, gt, St, sj);
                         touch |= hubo_touch<ORD>(x, inv, q);
-                    }
+                    });
                     touch = __reduce_or_sync(FULL, touch) & pend;
                     __syncwarp();
                     if (touch) {
@@ -168,7 +184,7 @@ __device__ __noinline__ int hubo_sweep(const int *hptr, const int4 *hrec, uint32
 
 // One worldline sweep, whole CTA (ends with a barrier); the number of moves.
 template <bool ORD>
-__device__ __noinline__ int hubo_worldlines(const int *hptr, const int4 *hrec, uint32_t ordo, int n, int NP, float B,
+__device__ __noinline__ int hubo_worldlines(const HubRows hr, uint32_t ordo, int n, int NP, float B,
                                             uint64_t key, uint32_t slot, uint32_t sigma) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, W = blockDim.x >> 5;
     const int nw = (n + 31) >> 5, n32 = nw * 32, ld = dense_ld(n);
@@ -221,15 +237,15 @@ __device__ __noinline__ int hubo_worldlines(const int *hptr, const int4 *hrec, u
         const int ws = __ffs(with) - 1;
         if (warp == ws) {
             // the moves before the first lane that one of them changes
-            const int c0 = __ldg(hptr + i), c1 = __ldg(hptr + i + 1);
+            const uint4 hs = __ldg(hr.spin + i);
             uint32_t F = 0, T = 0;
             for (uint32_t mm = m; mm; mm &= mm - 1u) {
                 const int j = __ffs(mm) - 1;
                 if (T && __ffs(T) - 1 <= j) break;
                 F |= 1u << j;
-                const int a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
-                uint32_t touch = 0;
-                for (int c = a; c < b; ++c) touch |= hubo_touch<ORD>(__ldg(hrec + 32 * c + lane), inv, q);
+                const uint4 hj = hub_of(hs, j);
+                uint32_t touch = hubo_touch<ORD>(hub_first(hr, hj.x, hj.y, lane), inv, q);
+                hub_chunks(hj, hr.off, hr.rec, lane, [&](const int4 &x) { touch |= hubo_touch<ORD>(x, inv, q); });
                 T |= __reduce_or_sync(FULL, touch) & (j == 31 ? 0u : ~((2u << j) - 1u));
             }
             wsp[lane] = i;
@@ -241,20 +257,19 @@ __device__ __noinline__ int hubo_worldlines(const int *hptr, const int4 *hrec, u
         __syncthreads();
         const uint32_t F = (uint32_t)flag[1];
         const int again = flag[2], isp = wsp[lane];
-        const int c0 = __ldg(hptr + isp), c1 = __ldg(hptr + isp + 1);
+        const uint4 hs = __ldg(hr.spin + isp);
         for (int t = warp; t < NP; t += W) {
             uint32_t *St = S + t * nw;
             for (uint32_t f = F; f; f &= f - 1u) {
                 const int j = __ffs(f) - 1, jj = __shfl_sync(FULL, isp, j);
-                const int a = __shfl_sync(FULL, c0, j), b = __shfl_sync(FULL, c1, j);
+                const uint4 hj = hub_of(hs, j);
+                const int4 rec = hub_first(hr, hj.x, hj.y, lane);
                 const int sj = -spin_of(St, jj);
                 __syncwarp();
                 if (lane == 0) St[jj >> 5] ^= 1u << (jj & 31);
-                for (int c = a; c < b; ++c) {
-                    const int4 x = __ldg(hrec + 32 * c + lane);
-                    __syncwarp();
-                    hubo_add(x, G + t * ld, St, sj);
-                }
+                __syncwarp();
+                hubo_add(rec, G + t * ld, St, sj);
+                hub_chunks(hj, hr.off, hr.rec, lane, [&](const int4 &x) { hubo_add(x, G + t * ld, St, sj); });
                 __syncwarp();
             }
         }
@@ -277,8 +292,7 @@ __global__ void __launch_bounds__(512, 1) ring_hubo_kernel(RingParams p) {
     const ProbDev *Pd = p.probs + R.prob;
     const int NP = p.P, W = p.W, n = Pd->n, nw = Pd->nw, n32 = nw * 32, ld = dense_ld(n), T = Pd->T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int *hptr = Pd->hub_ptr;
-    const int4 *hrec = Pd->hub_rec;
+    const HubRows hr{Pd->hub_spin, Pd->hub_off, Pd->hub_rec};
     const HuboLay L = hubo_layout(NP, n, ORD);
     float *G = dsm<float>(L.G), *h = dsm<float>(L.h);
     uint32_t *S = dsm<uint32_t>(L.S);
@@ -323,13 +337,13 @@ __global__ void __launch_bounds__(512, 1) ring_hubo_kernel(RingParams p) {
             const uint32_t sigma = (uint32_t)(step * p.spb + sw), tag = p.slice_tag | R.tag_extra;
             const uint32_t ord = begin_sweep();
             if (ORD) {
-                acc_s += (unsigned long long)hubo_sweep<true>(hptr, hrec, ord, p.counters + 4, n, NP, warp, NP, W, B, T4,
+                acc_s += (unsigned long long)hubo_sweep<true>(hr, ord, p.counters + 4, n, NP, warp, NP, W, B, T4,
                                                               R.key, (uint32_t)(slot * NP), sigma, tag);
                 __syncthreads();
             } else {
                 for (int ph = 0; ph < 3; ++ph) {
                     const int cnt = phase_count(NP, ph), b = phase_slice(NP, ph, 0);
-                    acc_s += (unsigned long long)hubo_sweep<false>(hptr, hrec, 0, nullptr, n, NP, b + 2 * warp,
+                    acc_s += (unsigned long long)hubo_sweep<false>(hr, 0, nullptr, n, NP, b + 2 * warp,
                                                                    b + 2 * cnt, 2 * W, B, T4, R.key,
                                                                    (uint32_t)(slot * NP), sigma, tag);
                     if (cnt) __syncthreads();
@@ -354,7 +368,7 @@ __global__ void __launch_bounds__(512, 1) ring_hubo_kernel(RingParams p) {
         for (int sw = 0; sw < wls; ++sw) {
             const uint32_t sigma = (uint32_t)(step * p.wls + sw);
             const uint32_t ord = begin_sweep();
-            const int mv = hubo_worldlines<ORD>(hptr, hrec, ord, n, NP, B, R.key, (uint32_t)slot, sigma);
+            const int mv = hubo_worldlines<ORD>(hr, ord, n, NP, B, R.key, (uint32_t)slot, sigma);
             if (threadIdx.x == 0) {
                 att_w += (unsigned long long)n;
                 acc_w += (unsigned long long)mv;
