@@ -1602,15 +1602,16 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
     bool small_terms = true;
     for (int t = 0; t < n_terms && small_terms; ++t) small_terms = tptr[t + 1] - tptr[t] <= 4;
     std::vector<uint4> hub_spin;
-    std::vector<uint32_t> hub_off;
+    std::vector<uint32_t> hub_size;
     std::vector<int4> hub_rec;
     if (small_terms) {
         hub_spin.assign(n, make_uint4(0u, 0u, 0u, 0u));
-        hub_off.assign(1, 0u);
         struct U { int v, t, w1, w2; };
         std::vector<U> u;
         std::vector<std::pair<int, int>> runs;  // the records of each target: (first, number)
-        std::vector<uint32_t> chunk_of(n, 0u);  // the last chunk (counted from 1) with the target
+        std::vector<uint32_t> size;               // of the spin's chunks
+        std::vector<uint32_t> chunk_of(n, 0u);    // the last chunk with the target, chunks counted from 1
+        uint32_t chunk = 0;
         for (int j = 0; j < n; ++j) {
             u.clear();
             for (int q = incptr[j]; q < incptr[j + 1]; ++q) {
@@ -1634,31 +1635,37 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
             // the first record of every target, then the second, ..; targets with the
             // most records first, so that a chunk can run on into the next round
             std::stable_sort(runs.begin(), runs.end(), [](const auto &a, const auto &b) { return a.second > b.second; });
-            const uint32_t c0 = (uint32_t)hub_off.size();  // this spin's first chunk, counted from 1
-            uint32_t in_chunk = 0;
+            const uint32_t first = (uint32_t)hub_rec.size();
+            size.assign(1, 0u);
+            ++chunk;
             size_t left = runs.size();
             for (int round = 0; left > 0; ++round) {
                 while (left > 0 && runs[left - 1].second <= round) --left;
                 for (size_t r = 0; r < left; ++r) {
                     const U &x = u[(size_t)(runs[r].first + round)];
-                    if (in_chunk == 32 || chunk_of[x.v] == (uint32_t)hub_off.size()) {
-                        hub_off.push_back((uint32_t)hub_rec.size());
-                        in_chunk = 0;
+                    if (size.back() == 32u || chunk_of[x.v] == chunk) {
+                        size.push_back(0u);
+                        ++chunk;
                     }
-                    chunk_of[x.v] = (uint32_t)hub_off.size();
+                    chunk_of[x.v] = chunk;
                     const float two = 2.0f * c32[x.t];
                     int bits;
                     std::memcpy(&bits, &two, 4);
                     hub_rec.push_back(make_int4(x.v, x.w1, x.w2, bits));
-                    ++in_chunk;
+                    ++size.back();
                 }
             }
-            hub_off.push_back((uint32_t)hub_rec.size());
-            const uint32_t chunks = (uint32_t)hub_off.size() - c0;
-            uint32_t sizes = 0;
-            for (uint32_t k = 0; k < std::min(4u, chunks); ++k)
-                sizes |= (hub_off[c0 + k] - hub_off[c0 + k - 1]) << (8 * k);
-            hub_spin[j] = make_uint4(hub_off[c0 - 1], sizes, c0 + 3, std::max(c0 + 3, c0 + chunks - 1));
+            size.resize((size.size() + 3) / 4 * 4, 0u);
+            const uint32_t words = (uint32_t)hub_size.size();
+            uint32_t first_four = 0;
+            for (size_t k = 0; k < size.size(); k += 4) {
+                const uint32_t w = size[k] | size[k + 1] << 8 | size[k + 2] << 16 | size[k + 3] << 24;
+                if (k == 0)
+                    first_four = w;
+                else
+                    hub_size.push_back(w);
+            }
+            hub_spin[j] = make_uint4(first, first_four, words, (uint32_t)hub_size.size());
         }
     }
     qa_problem *P = new qa_problem();
@@ -1677,7 +1684,7 @@ int qa_problem_hubo(qa_ctx *ctx, int n, const double *h, int n_terms, const int6
     if (rc == QA_OK) rc = upload(P, coeff, (size_t)n_terms, &P->dev.coef64);
     if (rc == QA_OK && small_terms) {
         rc = upload(P, hub_spin.data(), hub_spin.size(), &P->dev.hub_spin);
-        if (rc == QA_OK) rc = upload(P, hub_off.data(), hub_off.size(), &P->dev.hub_off);
+        if (rc == QA_OK) rc = upload(P, hub_size.data(), hub_size.size(), &P->dev.hub_size);
         if (rc == QA_OK) rc = upload(P, hub_rec.data(), hub_rec.size(), &P->dev.hub_rec);
         // one 16-byte record per term for the per-step energy scan
         std::vector<int4> trec(std::max(n_terms, 1), make_int4(-1, -1, -1, -1));

@@ -151,14 +151,15 @@ struct ProbDev {
     // bits J[m][32q .. 32q+31] (1 = +1; diagonal and padding bits 0); else null
     const uint32_t *Jw;
     // hubo with every term of degree <= 4: the field updates of a flip of
-    // spin j in chunks of up to 32 records (one load of a warp), chunk c =
-    // hub_rec[hub_off[c] .. hub_off[c+1]).  Record {v, w1, w2, bits(2 J_t)}: target
-    // v, w1, w2 the term's other spins (-1: none).  A chunk holds a target once; a
-    // target's terms stand in increasing order, one chunk after another.
-    // hub_spin[j] = {first record, the sizes of the first four chunks in a byte each,
-    // first and end of the chunks after those}.  Else null.
+    // spin j in chunks of up to 32 records of hub_rec (one load of a warp), one
+    // chunk behind the other.  Record {v, w1, w2, bits(2 J_t)}: target v, w1, w2 the
+    // term's other spins (-1: none).  A chunk holds a target once; a target's
+    // terms stand in increasing order, one chunk after another.  hub_spin[j] =
+    // {first record, the sizes of the first four chunks in a byte each (0: no
+    // chunk), first and end of the words of hub_size with those of the others}.
+    // Else null.
     const uint4 *hub_spin;
-    const uint32_t *hub_off;
+    const uint32_t *hub_size;
     const int4 *hub_rec;
     // hubo with every term of degree <= 4: term t's spins {v0, v1, v2, v3}
     // (-1: none) in one 16-byte record, for the per-step energy scan; else null
@@ -173,46 +174,49 @@ struct ProbDev {
 };
 
 __device__ __forceinline__ int spin_of(const uint32_t *S, int i) { return ((S[i >> 5] >> (i & 31)) & 1u) ? 1 : -1; }
+// 1 when spin v of the bits S is down (-1).
+__device__ __forceinline__ uint32_t down_bit(const uint32_t *S, int v) { return ~(S[v >> 5] >> (v & 31)) & 1u; }
 
 // f on this lane's record (x < 0: none) of each chunk after the first of a spin with
 // hub_spin entry hs (the same in all lanes), in order, the warp in step before each; up
-// to four chunks' loads in flight.
+// to four chunks' loads in flight.  (The first four apart: one loop over all of them
+// costs models of one chunk a spin 7% of ring_kernel<K_HUBO> at n = 64.)
 template <class F>
-__device__ __forceinline__ void hub_chunks(const uint4 &hs, const uint32_t *off, const int4 *rec, int lane, F f) {
-    const uint32_t size = hs.y >> 8;
-    if (size == 0u) return;
-    const int4 none = make_int4(-1, -1, -1, 0);
-    int4 r[4];
-    uint32_t at = hs.x + (hs.y & 255u);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const uint32_t c = (size >> (8 * k)) & 255u;
-        r[k] = (uint32_t)lane < c ? __ldg(rec + at + lane) : none;
-        at += c;
-    }
-#pragma unroll
-    for (int k = 0; k < 3; ++k)
-        if ((size >> (8 * k)) & 255u) {
-            __syncwarp();
-            f(r[k]);
-        }
-#pragma unroll 1
-    for (uint32_t c = hs.z; c < hs.w; c += 4) {
+__device__ __forceinline__ void hub_chunks(const uint4 &hs, const uint32_t *sizes, const int4 *rec, int lane, F f) {
+    if (hs.y < 256u) return;
+    uint32_t at = hs.x + (hs.y & 255u), size = hs.y >> 8;
+    auto four = [&]() {
+        int4 r[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            r[k] = none;
-            if (c + k < hs.w) {
-                const uint32_t a = __ldg(off + c + k) + (uint32_t)lane;
-                if (a < __ldg(off + c + k + 1)) r[k] = __ldg(rec + a);
-            }
+            const uint32_t s = (size >> (8 * k)) & 255u;
+            r[k] = (uint32_t)lane < s ? __ldg(rec + at + lane) : make_int4(-1, -1, -1, 0);
+            at += s;
         }
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-            if (c + k < hs.w) {
+            if ((size >> (8 * k)) & 255u) {
                 __syncwarp();
                 f(r[k]);
             }
+    };
+    four();
+#pragma unroll 1
+    for (uint32_t c = hs.z; c < hs.w; ++c) {
+        size = __ldg(sizes + c);
+        four();
     }
+}
+
+// One record's update after a flip of its spin (new value sj = +-1): S holds the
+// flip.
+__device__ __forceinline__ void hub_add(const int4 &r, float *g, const uint32_t *S, int sj) {
+    if (r.x < 0) return;
+    uint32_t down = sj < 0 ? 1u : 0u;
+    if (r.y >= 0) down ^= down_bit(S, r.y);
+    if (r.z >= 0) down ^= down_bit(S, r.z);
+    const float two = __int_as_float(r.w);
+    g[r.x] = __fadd_rn(g[r.x], down ? -two : two);
 }
 
 // Field update after spin j (old value so) flipped in one slice whose spin bits
@@ -238,16 +242,8 @@ __device__ __forceinline__ void apply_flip(const ProbDev &P, float *g, const uin
         // additions, in the same order per field, as the term-by-term loop
         const int sj = spin_of(S, j);  // S holds the new spin
         const uint4 hs = __ldg(P.hub_spin + j);
-        auto add = [&](const int4 &rc) {
-            if (rc.x < 0) return;
-            int pr = sj;
-            if (rc.y >= 0) pr *= spin_of(S, rc.y);
-            if (rc.z >= 0) pr *= spin_of(S, rc.z);
-            const float two = __int_as_float(rc.w);
-            g[rc.x] = __fadd_rn(g[rc.x], pr > 0 ? two : -two);
-        };
-        if ((uint32_t)lane < (hs.y & 255u)) add(__ldg(P.hub_rec + hs.x + lane));
-        hub_chunks(hs, P.hub_off, P.hub_rec, lane, add);
+        if ((uint32_t)lane < (hs.y & 255u)) hub_add(__ldg(P.hub_rec + hs.x + lane), g, S, sj);
+        hub_chunks(hs, P.hub_size, P.hub_rec, lane, [&](const int4 &r) { hub_add(r, g, S, sj); });
     } else {
         const int q0 = __ldg(P.incptr + j), q1 = __ldg(P.incptr + j + 1);
         for (int q = q0; q < q1; ++q) {
@@ -341,9 +337,6 @@ __device__ __forceinline__ double cell_energy(const ProbDev &P, const uint32_t *
     pj = warp_sum_d(pj);
     return __dadd_rn(P.c, __dadd_rn(ph, pj));
 }
-
-// 1 when spin v of the bits S is down (-1).
-__device__ __forceinline__ uint32_t down_bit(const uint32_t *S, int v) { return ~(S[v >> 5] >> (v & 31)) & 1u; }
 
 // cell_energy<K_HUBO> of two slices Sa, Sb in one pass over the term records:
 // every term's sign is the parity of its down spins.  Each slice's sums take

@@ -59,10 +59,10 @@ __host__ __device__ inline size_t hubo_smem_bytes(int P, int n, bool ref_order) 
     return hubo_layout(P, n, ref_order).total;
 }
 
-// The field updates of a flip (ProbDev::hub_spin, hub_off, hub_rec).
+// The field updates of a flip (ProbDev::hub_spin, hub_size, hub_rec).
 struct HubRows {
     const uint4 *spin;
-    const uint32_t *off;
+    const uint32_t *size;
     const int4 *rec;
 };
 
@@ -73,17 +73,6 @@ __device__ __forceinline__ uint4 hub_of(const uint4 &hs, int j) {
 }
 __device__ __forceinline__ int4 hub_first(const HubRows &hr, uint32_t at, uint32_t sizes, int lane) {
     return (uint32_t)lane < (sizes & 255u) ? __ldg(hr.rec + at + lane) : make_int4(-1, -1, -1, 0);
-}
-
-// One record's update after a flip of its spin (new value sj = +-1): S holds the
-// flip.
-__device__ __forceinline__ void hubo_add(const int4 &r, float *g, const uint32_t *S, int sj) {
-    if (r.x < 0) return;
-    uint32_t down = sj < 0 ? 1u : 0u;
-    if (r.y >= 0) down ^= down_bit(S, r.y);
-    if (r.z >= 0) down ^= down_bit(S, r.z);
-    const float two = __int_as_float(r.w);
-    g[r.x] = __fadd_rn(g[r.x], down ? -two : two);
 }
 
 // The lanes of block q (positions) that hold record r's target.
@@ -153,11 +142,11 @@ __device__ __noinline__ int hubo_sweep(const HubRows hr, uint32_t ordo, unsigned
                     const int jn = (m & pend) ? __ffs(m & pend) - 1 : j;  // the likely next flip
                     const int4 recn = chunk(jn);
                     __syncwarp();
-                    hubo_add(rec, gt, St, sj);
+                    hub_add(rec, gt, St, sj);
                     uint32_t touch = hubo_touch<ORD>(rec, inv, q);
                     // (chunks in order: a target's terms stay in order)
-                    hub_chunks(hj, hr.off, hr.rec, lane, [&](const int4 &x) {
-                        hubo_add(x, gt, St, sj);
+                    hub_chunks(hj, hr.size, hr.rec, lane, [&](const int4 &x) {
+                        hub_add(x, gt, St, sj);
                         touch |= hubo_touch<ORD>(x, inv, q);
                     });
                     touch = __reduce_or_sync(FULL, touch) & pend;
@@ -245,7 +234,7 @@ __device__ __noinline__ int hubo_worldlines(const HubRows hr, uint32_t ordo, int
                 F |= 1u << j;
                 const uint4 hj = hub_of(hs, j);
                 uint32_t touch = hubo_touch<ORD>(hub_first(hr, hj.x, hj.y, lane), inv, q);
-                hub_chunks(hj, hr.off, hr.rec, lane, [&](const int4 &x) { touch |= hubo_touch<ORD>(x, inv, q); });
+                hub_chunks(hj, hr.size, hr.rec, lane, [&](const int4 &x) { touch |= hubo_touch<ORD>(x, inv, q); });
                 T |= __reduce_or_sync(FULL, touch) & (j == 31 ? 0u : ~((2u << j) - 1u));
             }
             wsp[lane] = i;
@@ -268,8 +257,8 @@ __device__ __noinline__ int hubo_worldlines(const HubRows hr, uint32_t ordo, int
                 __syncwarp();
                 if (lane == 0) St[jj >> 5] ^= 1u << (jj & 31);
                 __syncwarp();
-                hubo_add(rec, G + t * ld, St, sj);
-                hub_chunks(hj, hr.off, hr.rec, lane, [&](const int4 &x) { hubo_add(x, G + t * ld, St, sj); });
+                hub_add(rec, G + t * ld, St, sj);
+                hub_chunks(hj, hr.size, hr.rec, lane, [&](const int4 &x) { hub_add(x, G + t * ld, St, sj); });
                 __syncwarp();
             }
         }
@@ -292,7 +281,7 @@ __global__ void __launch_bounds__(512, 1) ring_hubo_kernel(RingParams p) {
     const ProbDev *Pd = p.probs + R.prob;
     const int NP = p.P, W = p.W, n = Pd->n, nw = Pd->nw, n32 = nw * 32, ld = dense_ld(n), T = Pd->T;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const HubRows hr{Pd->hub_spin, Pd->hub_off, Pd->hub_rec};
+    const HubRows hr{Pd->hub_spin, Pd->hub_size, Pd->hub_rec};
     const HuboLay L = hubo_layout(NP, n, ORD);
     float *G = dsm<float>(L.G), *h = dsm<float>(L.h);
     uint32_t *S = dsm<uint32_t>(L.S);
