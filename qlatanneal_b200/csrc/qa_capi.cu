@@ -754,9 +754,12 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
     pl->hubo = !clusters && kind == K_HUBO && P <= 64 && !std::getenv("QA_DISABLE_HUBO") &&
                hubo_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin;
     for (int p = 0; p < np && pl->hubo; ++p) pl->hubo = probs[p]->dev.hub_rec != nullptr;
+    const int hubo_w = hubo_warps(P, n_rings, ctx->sms, ref_order, hubo_smem_bytes(P, n_max, ref_order),
+                                  (size_t)ctx->smem_optin);
+    pl->hubo = pl->hubo && hubo_w > 0;
     if (pl->hubo) {
         pl->smem = hubo_smem_bytes(P, n_max, ref_order);
-        if (ctx->tune.warps_per_ring <= 0) pl->W = std::min(P, 16);
+        if (ctx->tune.warps_per_ring <= 0) pl->W = hubo_w;
         pl->W = std::min(pl->W, 16);
         return QA_OK;
     }

@@ -59,6 +59,36 @@ __host__ __device__ inline size_t hubo_smem_bytes(int P, int n, bool ref_order) 
     return hubo_layout(P, n, ref_order).total;
 }
 
+// Warps of a ring (at most 16: up to 126 registers a thread), 0 for ring_kernel.  smem: a
+// ring's shared memory, cap: an SM's.
+// qanneal's order: w warps take P / w slices each, behind one another; more rings an SM
+// against a longer share, by waves of rings times P / w + 2.6 (fits n = 24 .. 200, P = 1
+// .. 64, 148 .. 3000 rings within 1% of the best w on average: P = 16, n = 64, 450 rings 4
+// warps 1.9 times as fast as 16).
+// Checkerboard: where the slices of a phase fit on the SMs, 16 warps each, a warp for
+// each (1.2 to 1.5 times ring_kernel); where they do not, ring_kernel with its 64
+// registers is faster at every n (n = 200: P = 16, 600 rings 0.90, P = 24, 200 rings
+// 0.86, P = 64, 100 rings 0.93 of its speed here; but P = 16, 200 rings 1.35).
+inline int hubo_warps(int P, int rings, int sms, bool ref_order, size_t smem, size_t cap) {
+    const int most = std::min(P, 16), phase = (P + 1) / 2;
+    if (!ref_order || P == 1) {
+        if (rings > sms * (16 / phase)) return 0;
+        return rings > sms ? std::min(most, phase) : most;
+    }
+    const int fit = std::max(1, (int)(cap / smem));
+    int best = most;
+    double cost = 0.0;
+    for (int w = most; w >= 1; --w) {
+        const int per_sm = std::min(16 / w, fit);
+        const double c = std::ceil((double)rings / ((double)per_sm * sms)) * ((double)P / w + 2.6);
+        if (w == most || c < cost) {
+            best = w;
+            cost = c;
+        }
+    }
+    return best;
+}
+
 // The field updates of a flip (ProbDev::hub_spin, hub_size, hub_rec).
 struct HubRows {
     const uint4 *spin;

@@ -35,6 +35,15 @@ def dense_checkerboard(n, P, reads):
     return ann, lambda: ann.run_reads(3, 0, reads=reads, seed=1)
 
 
+def hubo_rings(n, P, reads, order):
+    """Pair terms on a ring: little to do at a flip, many rings."""
+    qa.set_update_order(order)
+    terms = {tuple(sorted((i, (i + 1) % n))): 1.0 - 2.0 * (i % 3 == 0) for i in range(n)}
+    ann = qa.SQAAnnealer(qa.HigherOrderIsing(terms, n), qa.SQASchedule.from_vectors(
+        P * np.linspace(0.1, 2.0, 6), np.linspace(2.0, 0.05, 6)), P)
+    return ann, lambda: ann.run_reads(2, 0, reads=reads, seed=1)
+
+
 SHAPES = [
     (sa_real, "QA_DISABLE_DENSE", (24, 4000)),
     (sa_real, "QA_DISABLE_DENSE", (64, 2000)),
@@ -48,6 +57,9 @@ SHAPES = [
     (dense_checkerboard, "QA_DISABLE_DENSE", (24, 12, 600)),
     (dense_checkerboard, "QA_DISABLE_DENSE", (64, 5, 1000)),
     (dense_checkerboard, "QA_DISABLE_DENSE", (200, 8, 600)),
+    (hubo_rings, "QA_DISABLE_HUBO", (200, 16, 600, "checkerboard")),
+    (hubo_rings, "QA_DISABLE_HUBO", (64, 8, 1000, "checkerboard")),
+    (hubo_rings, "QA_DISABLE_HUBO", (200, 4, 600, "reference")),
 ]
 
 
