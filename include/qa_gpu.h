@@ -92,8 +92,11 @@ QA_API int qa_get_update_order(const qa_ctx *ctx, int *order);
 /* Launch-shape overrides of a context, for the autotuner (no counterpart in
  * the reference: its loops have no launch shape).  Every choice leaves the
  * results unchanged bit for bit; it moves only time.  0 / -1 is automatic.
- *   warps_per_ring: warps of a ring's CTA (1..32, at most P; automatic:
- *                   ceil(P/2));
+ *   warps_per_ring: warps of a ring's CTA (1..32, at most P; the kernels of
+ *                   dense real couplings and of terms of at most four spins
+ *                   take at most 16, that of sparse neighbour records at most
+ *                   8, which there may exceed P; automatic: by kernel, slices,
+ *                   spins and rings, see qa_ring_warps);
  *   field_form:     the dense +-1 kernel's ring state: 0 int32 fields and the
  *                   coupling bits in shared memory, 1 int16 fields and the
  *                   bits in shared memory, 2 int16 fields and the bits read
@@ -113,6 +116,12 @@ typedef struct {
 } qa_tuning;
 QA_API int qa_set_tuning(qa_ctx *ctx, const qa_tuning *tuning);  /* NULL: all automatic */
 QA_API int qa_get_tuning(const qa_ctx *ctx, qa_tuning *tuning);
+/* The warps of a ring's CTA that a run of these problems takes under the
+ * context's present overrides and update order: trotter_slices slices, `rings`
+ * rings in all; checkerboard != 0 for SQA-Chi, clusters != 0 with cluster
+ * sweeps.  Nothing is launched. */
+QA_API int qa_ring_warps(qa_ctx *ctx, const qa_problem *const *problems, int n_problems, int trotter_slices, int rings,
+                         int checkerboard, int clusters, int *warps);
 
 /* ---- problems (device copies of one model instance) ------------------- */
 

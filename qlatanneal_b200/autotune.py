@@ -17,7 +17,8 @@ environment variable QA_TUNE_CACHE) makes later runs of the SQA, SQA-PT,
 SQA-Chi and instance-set paths apply the cached shape of their bucket; the
 runs a tuning times keep their candidate shape.
 
-The search is coordinate-wise: warps per ring, then the ring-state form (dense
+The search is coordinate-wise: warps per ring (candidates that a kernel's
+limit makes the same launch are timed once), then the ring-state form (dense
 models), then rotation (off, or on with steps 25 / 50 / 100 and groups of 2 /
 3 / 4 rings when the rings outnumber the SMs); each stage keeps the previous
 stages' winners.
@@ -122,10 +123,33 @@ def _signature(res) -> tuple:
     return tuple((float(r.best_energy), bytes(r.best_state.as_array().tobytes())) for r in res)
 
 
-def _tune(key: str, run, kind: str, P: int, rings: int, cache_path: Optional[str], repeats: int = 2,
-          device: Optional[int] = None) -> dict:
+def _ring_warps(eng, model, P: int, rings: int, checkerboard: bool, clusters: bool) -> int:
+    """Warps of a ring's CTA under the context's present shape."""
+    w = C.c_int()
+    probs = (C.c_void_p * 1)(model._device_problem(eng))
+    _lib.check(eng.L.qa_ring_warps(eng.h, probs, 1, int(P), int(rings), int(checkerboard), int(clusters), C.byref(w)))
+    return w.value
+
+
+def _distinct(cands: List[dict], warps_of, seen: set) -> List[dict]:
+    """The candidates whose launch has a number of warps not in ``seen`` yet."""
+    out = []
+    for c in cands:
+        w = warps_of(c)
+        if w not in seen:
+            seen.add(w)
+            out.append(c)
+    return out
+
+
+def _tune(key: str, run, model, kind: str, P: int, rings: int, cache_path: Optional[str], repeats: int = 2,
+          device: Optional[int] = None, clusters: bool = False) -> dict:
     eng = _lib.Engine.get(device)
     sms = _sm_count()
+
+    def warps_of(tuning):
+        set_tuning(eng, tuning)
+        return _ring_warps(eng, model, P, rings, kind.endswith("-chi"), clusters)
 
     def timed(tuning):
         set_tuning(eng, tuning)
@@ -144,7 +168,10 @@ def _tune(key: str, run, kind: str, P: int, rings: int, cache_path: Optional[str
     auto_ms, ref_sig = timed(base)
     best_ms, tried = auto_ms, [dict(tuning=dict(base), ms=auto_ms)]
     for stage in ("warps", "form", "rotation"):
-        for cand in _candidates_stage(stage, base, kind, P, rings, sms):
+        cands = _candidates_stage(stage, base, kind, P, rings, sms)
+        if stage == "warps":
+            cands = _distinct(cands, warps_of, {warps_of(base)})
+        for cand in cands:
             ms, sig = timed(cand)
             if sig != ref_sig:
                 set_tuning(eng, None)
@@ -195,7 +222,8 @@ def tune_sqa(annealer, sweeps_per_beta: int, worldline_sweeps: int, reads: int, 
 
     rings = reads * annealer.replicas
     key = bucket(m.kind, m.size(), annealer.trotter_slices, rings)
-    return _tune(key, run, m.kind, annealer.trotter_slices, rings, cache_path, device=annealer.device)
+    return _tune(key, run, m, m.kind, annealer.trotter_slices, rings, cache_path, device=annealer.device,
+                 clusters=cluster_sweeps > 0)
 
 
 def tune_sqapt(annealer, sweeps_per_step: int, worldline_sweeps: int, steps: int, swap_interval: int, reads: int,
@@ -213,7 +241,8 @@ def tune_sqapt(annealer, sweeps_per_step: int, worldline_sweeps: int, steps: int
     m = annealer.hamiltonian
     rings = reads * len(annealer.betas)
     key = bucket(m.kind, m.size(), annealer.trotter_slices, rings)
-    return _tune(key, run, m.kind, annealer.trotter_slices, rings, cache_path, device=annealer.device)
+    return _tune(key, run, m, m.kind, annealer.trotter_slices, rings, cache_path, device=annealer.device,
+                 clusters=cluster_sweeps > 0)
 
 
 def tune_chi(annealer, reads: int, timing_steps: Optional[int] = None, cache_path: Optional[str] = None,
@@ -235,4 +264,4 @@ def tune_chi(annealer, reads: int, timing_steps: Optional[int] = None, cache_pat
     kind = m.kind + "-chi"
     rings = reads * annealer.replicas
     key = bucket(kind, m.size(), annealer.trotter_slices, rings)
-    return _tune(key, run, kind, annealer.trotter_slices, rings, cache_path, device=annealer.device)
+    return _tune(key, run, m, kind, annealer.trotter_slices, rings, cache_path, device=annealer.device)

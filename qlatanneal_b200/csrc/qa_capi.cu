@@ -725,7 +725,7 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
         pl->wide = P > 32;
         pl->smem = slab_smem_bytes(P, n_max, ref_order);
         pl->smem_fields = 0;
-        pl->W = std::min(8, (n_max + 127) / 128);
+        pl->W = std::min(8, ctx->tune.warps_per_ring > 0 ? ctx->tune.warps_per_ring : (n_max + 127) / 128);
         return QA_OK;
     }
     // sparse integer couplings: fields on demand, worldline sums from bits
@@ -1734,6 +1734,20 @@ int qa_set_tuning(qa_ctx *ctx, const qa_tuning *t) {
 int qa_get_tuning(const qa_ctx *ctx, qa_tuning *t) {
     if (!ctx || !t) return fail(QA_ERR_ARG, "null argument");
     *t = ctx->tune;
+    return QA_OK;
+}
+
+int qa_ring_warps(qa_ctx *ctx, const qa_problem *const *problems, int n_problems, int trotter_slices, int rings,
+                  int checkerboard, int clusters, int *warps) {
+    QA_TRY(begin(ctx));
+    if (!warps) return fail(QA_ERR_ARG, "null output pointer");
+    if (trotter_slices <= 0 || rings <= 0) return fail(QA_ERR_ARG, "trotter_slices and rings must be > 0.");
+    int kind, n_max;
+    QA_TRY(check_batch(problems, n_problems, &kind, &n_max));
+    RingPlan pl;
+    QA_TRY(plan_rings(ctx, problems, n_problems, kind, trotter_slices, n_max, &pl, rings, clusters != 0,
+                      !checkerboard && ctx->update_order == QA_ORDER_REFERENCE));
+    *warps = pl.W;
     return QA_OK;
 }
 
