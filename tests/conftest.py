@@ -25,3 +25,17 @@ def ref():
     if not os.path.exists(REF_SO):
         pytest.skip("the compiled reference (oracle/_ref) is not present")
     return Ref()
+
+
+def pytest_collection_modifyitems(items):
+    """The C++ binding's check program is built against qanneal's own headers.  Where
+    this tree has neither those nor a program built elsewhere, its tests cannot
+    run; a missing program where it could have been built stays a failure."""
+    program = os.path.join(ROOT, "tests", "cxx", "_build", "backend_check")
+    core = os.path.join(ROOT, "oracle", "_ref", "libqanneal_ref.so")
+    if os.path.exists(program) or os.path.exists(core):
+        return
+    skip = pytest.mark.skip(reason="tests/cxx/_build/backend_check is absent and qanneal's headers are not here to build it")
+    for item in items:
+        if os.path.basename(str(item.fspath)) == "test_gpu_cxx_backend.py":
+            item.add_marker(skip)
