@@ -122,6 +122,12 @@ __device__ __forceinline__ void st_release_cta64(unsigned long long *p, unsigned
     asm volatile("st.release.cta.shared.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "l"(v)
                  : "memory");
 }
+// Enough for a slice's progress: the word itself carries the new bits of the block in
+// work, pbits of a finished block precede a fence and a store for the next block, and
+// nothing else is handed on: no slice reads another's flips in the worldline words,
+// nor its fields, before the next CTA barrier.  Nor can the store pass the reads of the
+// next slice's old bits, which that slice may flip once it sees the word: the votes
+// that the word's count rests on have consumed them.
 __device__ __forceinline__ void st_relaxed_cta64(unsigned long long *p, unsigned long long v) {
     asm volatile("st.relaxed.cta.shared.b64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p)), "l"(v)
                  : "memory");

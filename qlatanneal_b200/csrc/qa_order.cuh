@@ -240,8 +240,14 @@ __device__ __forceinline__ void pipe_wait(const SlicePipe &pp, int tp, int q, in
 
 // Whole warp, block q of slice t finished.  fenced: the warp wrote state a
 // later slice reads (every lane fences its writes and the warp synchronises
-// first).  Every lane stores the count (release; the same value, one store
+// first; release).  Every lane stores the count (the same value, one store
 // instruction).
+// Not fenced (ring_pm1_kernel, blocks without flips): a relaxed store.  There the
+// slices hand on the worldline words alone, and their last write precedes the fence
+// of the block that made it; what the slice has written since, its own spin bits
+// and fields, no other slice reads before the next CTA barrier.  Nor can the store
+// pass the block's reads of the next slice's bits, which that slice may flip once it
+// sees the count: the vote that found no flip has consumed them.
 __device__ __forceinline__ void pipe_publish(const SlicePipe &pp, int t, int q, int lane, bool fenced = true) {
     (void)lane;
     if (fenced) {
@@ -250,7 +256,7 @@ __device__ __forceinline__ void pipe_publish(const SlicePipe &pp, int t, int q, 
     }
     if (fenced)
         st_release_cta(pp.prog + t, q + 1);
-    else  // the warp has written nothing since its last fence, which orders what came before
+    else
         asm volatile("st.relaxed.cta.shared.b32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(pp.prog + t)), "r"(q + 1)
                      : "memory");
 }
