@@ -704,14 +704,12 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
         // resident ring: P <= 16 (512 threads), a ring whose shared memory
         // leaves one CTA per SM anyway (measured: n=256/2048 P=16 and n=1024
         // P=32 8-26% faster, n=512 P=32 at two rings per SM 2-13% slower), or
-        // no more rings than SMs and enough blocks that half the warps would
-        // stall the wavefront (100 rings, (P + 1)/2 -> P warps: n=512 P=20
-        // 1.24, n=400 P=24 1.14, n=400 P=32 1.03, n=256 P=24 1.03 times as
-        // fast; with fewer blocks the further warps only cost: n=256 P=32
-        // 0.94, n=100 P=24 0.97, n=64 P=32 0.95)
+        // no more rings than SMs (whole runs, (P + 1)/2 -> P warps: n=512 P=32
+        // 100 rings 36.3 -> 29.3 ms, n=500 P=32 148 rings 43.8 -> 34.3, n=400
+        // P=18 140 rings 10.3 -> 7.8, n=256 P=24 140 rings 12.8 -> 10.4, n=100
+        // P=32 10 rings 10.1 -> 8.8, n=64 P=32 one ring 6.5 -> 5.7)
         if (ref_order && ctx->tune.warps_per_ring <= 0 && P <= 32 &&
-            (P <= 16 || (n_rings <= ctx->sms && 3 * ((n_max + 31) / 32) >= 2 * ((P + 1) / 2)) ||
-             2 * pl->smem > (size_t)ctx->smem_optin))
+            (P <= 16 || n_rings <= ctx->sms || 2 * pl->smem > (size_t)ctx->smem_optin))
             pl->W = P;
         return QA_OK;
     }
