@@ -32,8 +32,8 @@
 // What is left is the chain of votes: at n = 24 each further slice adds 0.26 us
 // (500 cycles) to a sweep.  Not kept: the couplings of a block in a shared-memory
 // tile (its gather cost what it saved), J in shared memory (48.7 against
-// 43.8 ms at n = 200, in an earlier form), 32 warps at 64 registers (spills:
-// 30 -> 48 ms), a shorter loop for blocks whose predecessor is done (the
+// 43.8 ms at n = 200, in an earlier form), 32 warps at 64 registers (30 -> 48 ms),
+// a shorter loop for blocks whose predecessor is done (the
 // chain, not the instruction count, is the time).
 #pragma once
 #include <algorithm>
@@ -230,8 +230,9 @@ __device__ __forceinline__ void dense_update_cols(const float *J, int ld, float 
 //   n = 280,  the same                                      20.8 -> 20.7 ms
 //   n = 1500, P = 16, 20 reads,  5 steps of 20 + 5          40.8 -> 33.0 ms
 // At most 256 fields keep the loop in line: the call costs there (n = 24
-// 10.9 -> 11.5 ms, n = 200 28.9 -> 31.5 ms), and both forms in one kernel spill.
-// Eight groups at a time spill too (n = 900 27.0 ms).
+// 10.9 -> 11.5 ms, n = 200 28.9 -> 31.5 ms).  Eight groups at a time: n = 900
+// 27.0 ms.  At 128 registers the kernels spill 16 to 56 bytes, the WIDE ones 164
+// to 264 around the calls and at most 12 inside a sweep.
 __device__ __noinline__ void dense_update_wide(const float *J, int ld, float *gt, uint32_t F, int i, uint32_t ups,
                                                int lane) {
     int base = 0;

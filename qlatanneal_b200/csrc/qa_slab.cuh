@@ -26,8 +26,9 @@
 // Bound by instruction issue: 122 warp instructions for 32 sites (585 before),
 // 2.3 issued a cycle and SM.  SQA-PT, n = 2048, P = 16, 1024 rings, device time of
 // 200 slice + 50 worldline sweeps: ring_sparse_kernel 144 -> 40.6 ms (58 -> 207 G
-// site attempts/s).  80 registers, three CTAs of 8 warps an SM: 128 registers
-// 54.1 against 52.1 ms for the call, 64 (spills) 64.1; 4 warps a ring the same.
+// site attempts/s).  80 registers, three CTAs of 8 warps an SM, about 200 bytes
+// spilled in slab_sweep: 128 registers 54.1 against 52.1 ms for the call, 64 (more
+// spilled) 64.1; 4 warps a ring the same.
 // Not kept: four slices at a time on one reading of the neighbours' words (a
 // ring's warps then follow four steps behind each other: 55 to 83 ms), sleeping
 // in the waits (no change).
