@@ -707,9 +707,12 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
         // no more rings than SMs (whole runs, (P + 1)/2 -> P warps: n=512 P=32
         // 100 rings 36.3 -> 29.3 ms, n=500 P=32 148 rings 43.8 -> 34.3, n=400
         // P=18 140 rings 10.3 -> 7.8, n=256 P=24 140 rings 12.8 -> 10.4, n=100
-        // P=32 10 rings 10.1 -> 8.8, n=64 P=32 one ring 6.5 -> 5.7)
+        // P=32 10 rings 10.1 -> 8.8, n=64 P=32 one ring 6.5 -> 5.7) and more than
+        // one block: a block of its own has no wavefront, and the further warps
+        // cost (n=5 P=32 30 rings 19.2 -> 20.5 ms, n=32 0.97 to 1.04 of the speed
+        // by P, n=40 1.02 to 1.14)
         if (ref_order && ctx->tune.warps_per_ring <= 0 && P <= 32 &&
-            (P <= 16 || n_rings <= ctx->sms || 2 * pl->smem > (size_t)ctx->smem_optin))
+            (P <= 16 || (n_rings <= ctx->sms && n_max > 32) || 2 * pl->smem > (size_t)ctx->smem_optin))
             pl->W = P;
         return QA_OK;
     }

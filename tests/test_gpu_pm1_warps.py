@@ -32,3 +32,11 @@ def test_few_and_many_rings_agree(oracle, n, P):
                 np.testing.assert_array_equal(np.asarray(res.energy_trace), trace)
     finally:
         oracle.set_update_order("reference")
+
+
+@pytest.mark.parametrize("n,P,warps", [(5, 32, 16), (32, 24, 12), (33, 24, 24), (32, 16, 16)])
+def test_one_block_has_no_wavefront(n, P, warps):
+    """Models of one block of 32 spins gain nothing from a warp for each slice."""
+    from qlatanneal_b200 import _lib, autotune
+    eng, model = _lib.Engine.get(None), qa.DenseIsing(*sk_dense(n, 1))
+    assert autotune._ring_warps(eng, model, P, 3, False, False) == warps
