@@ -73,19 +73,24 @@ __host__ __device__ inline size_t slab_smem_bytes(int P, int n, bool ref_order) 
 
 // Whether a call's rings run here or on ring_sparse_kernel.  A sweep is P slices one
 // after another for each 128 spins, so in the checkerboard order, where
-// ring_sparse_kernel sweeps P / 2 slices side by side, few spins and many slices are
-// faster there.  In units of one slice here (58 us of 50 sweeps) a sweep costs P;
-// there (n + 20) / 7.5, times what the rings share an SM's 32 such warps.  P = 32, one
-// ring, 50 slice sweeps: n = 40 0.64 / 1.74 ms there / here, n = 128 1.34 / 2.02,
-// n = 256 2.27 / 1.92; P = 16: n = 64 0.75 / 0.94, n = 128 1.20 / 1.01; P = 64, n = 40:
-// 148 rings 0.90 / 3.86, 600 rings 4.7 / 4.1.  In qanneal's order only one slice of one
-// block is faster there (n = 16, P = 1, one ring: 0.124 / 0.160 ms).
+// ring_sparse_kernel sweeps the slices of a phase side by side (two phases; three for
+// an odd P, one for P = 1), few spins and many slices are faster there.  In units of a
+// sixteenth of a slice here a sweep costs 16 (P + 2.5); there n + 24 a phase, times what
+// the rings share an SM's 32 such warps.  One ring or a few, there / here: P = 32, 50
+// slice sweeps: n = 40 0.64 / 1.74 ms, n = 128 1.34 / 2.02, n = 256 2.27 / 1.92; 40
+// steps: P = 16, n = 104 0.89 / 1.17; P = 8, n = 52 1.60 / 1.90; P = 4, n = 12 0.27 /
+// 0.38; P = 5, n = 40 2.01 / 1.25; P = 1, n = 14 0.114 / 0.162; many: P = 64, n = 40,
+// 148 rings 0.90 / 3.86, 600 rings 4.7 / 4.1.  In qanneal's order both take one slice
+// after another, and up to 13 spins are faster there (P = 20, n = 8, 14 rings 0.75 /
+// 1.07 ms; P = 16, n = 10, 2 rings 0.66 / 0.87; n = 16 from 0.91 to 1.2 times as fast
+// here).  2075 shapes, n = 8 .. 2000, 1 to 1500 rings, timed against
+// ring_sparse_kernel: with the lines here 13 below 0.96 of its speed, down to 0.81.
 inline bool slab_pays(int P, int n, int rings, int sms, bool ref_order) {
-    if (ref_order) return P > 1 || n > 32;
-    const int w = (P + 1) / 2, per_sm = std::max(1, 32 / w);
-    const double share = 1.0 + 1.5 * std::max(0.0, (double)rings / sms - 1.0) * w / 32.0;
-    const double waves = std::ceil((double)rings / ((double)per_sm * sms));
-    return (n + 20) * std::max(share, waves) > 7.5 * P;
+    const int w = (P + 1) / 2, per_sm = std::max(1, 32 / w), phases = P == 1 ? 1 : 2 + (P & 1);
+    const double share = std::max(1.0 + 1.5 * std::max(0.0, (double)rings / sms - 1.0) * w / 32.0,
+                                  std::ceil((double)rings / ((double)per_sm * sms)));
+    if (ref_order && P > 1) return n * share > 13.0;
+    return phases * (n + 24) * share > 16.0 * (P + 2.5);
 }
 
 __device__ __forceinline__ int popc_of(uint32_t w) { return __popc(w); }

@@ -27,6 +27,14 @@ def sparse_checkerboard(n, P, reads):
     return ann, lambda: ann.run_reads(5, 1, reads=reads, seed=1)
 
 
+def sparse_small(n, P, reads, order):
+    """A sweep a step: the energies of a step count as well."""
+    qa.set_update_order(order)
+    ann = qa.SQAAnnealer(qa.SparseIsing(*regular3(n, 1), n),
+                         qa.SQASchedule.from_vectors(P * np.linspace(0.1, 2.5, 40), np.linspace(2.0, 0.05, 40)), P)
+    return ann, lambda: ann.run_reads(1, 0, reads=reads, seed=1)
+
+
 def dense_checkerboard(n, P, reads):
     """Many rings: the slices of a phase at work on all SMs, not the chain of one."""
     qa.set_update_order("checkerboard")
@@ -53,6 +61,11 @@ SHAPES = [
     (sparse_checkerboard, "QA_DISABLE_SLAB", (128, 64, 32)),
     (sparse_checkerboard, "QA_DISABLE_SLAB", (512, 32, 32)),
     (sparse_checkerboard, "QA_DISABLE_SLAB", (128, 16, 600)),
+    (sparse_small, "QA_DISABLE_SLAB", (104, 16, 44, "checkerboard")),
+    (sparse_small, "QA_DISABLE_SLAB", (20, 8, 700, "checkerboard")),
+    (sparse_small, "QA_DISABLE_SLAB", (14, 1, 1, "checkerboard")),
+    (sparse_small, "QA_DISABLE_SLAB", (8, 20, 14, "reference")),
+    (sparse_small, "QA_DISABLE_SLAB", (10, 16, 2, "reference")),
     (dense_checkerboard, "QA_DISABLE_DENSE", (12, 8, 3000)),
     (dense_checkerboard, "QA_DISABLE_DENSE", (24, 12, 600)),
     (dense_checkerboard, "QA_DISABLE_DENSE", (64, 5, 1000)),
