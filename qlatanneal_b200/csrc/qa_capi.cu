@@ -743,7 +743,8 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
     pl->dense = !clusters && kind == K_DENSE && P <= 64 && !std::getenv("QA_DISABLE_DENSE") &&
                 dense_smem_bytes(P, n_max, ref_order) <= (size_t)ctx->smem_optin;
     for (int p = 0; p < np && pl->dense; ++p) pl->dense = probs[p]->plain_j;
-    const int dense_w = dense_warps(P, n_max, n_rings, ctx->sms, ref_order);
+    const int dense_w = dense_warps(P, n_max, n_rings, ctx->sms, ref_order, dense_smem_bytes(P, n_max, ref_order),
+                                    (size_t)ctx->smem_optin);
     pl->dense = pl->dense && dense_w > 0;
     if (pl->dense) {
         pl->smem = dense_smem_bytes(P, n_max, ref_order);

@@ -37,6 +37,7 @@
 // chain, not the instruction count, is the time).
 #pragma once
 #include <algorithm>
+#include <cmath>
 
 #include "qa_pm1.cuh"
 
@@ -91,17 +92,33 @@ __host__ __device__ inline size_t dense_smem_bytes(int P, int n, bool ref_order)
 // two rings on an SM then beat one with twice the warps (P = 32, 600 rings: n = 24
 // 23.3 -> 17.7 ms, n = 64 36.8 -> 28.3, n = 200 69.9 -> 66.4; 300 rings of n = 900
 // 25.1 -> 28.2, so not there).  In the checkerboard order half the slices rest: with
-// more rings than SMs no more warps than slices of a phase (18 slice sweeps, P = 8:
-// n = 200, 1000 rings 1.47 -> 0.92 ms; n = 24, 450 rings 0.195 -> 0.119), and with at
-// most two blocks nothing is left of the shorter chain where those no longer fit on the
-// SMs, 16 warps each: ring_kernel has 64 registers (n = 24: P = 8, 3000 rings 0.56 here
-// with 4 warps / 0.46 there; P = 24, 300 rings 0.35 / 0.29).
-inline int dense_warps(int P, int n, int rings, int sms, bool ref_order) {
+// more rings than SMs no more warps than slices of a phase, and of those the number
+// with the least waves of rings times rounds of a phase's slices (0.4: the rest of a
+// sweep in rounds; 350 shapes of n = 66 .. 400, P = 3 .. 48, 160 to 1200 rings: 1% from
+// the best number on average, 10% with 8 or a phase's slices for all; n = 84, P = 20,
+// 371 rings, 60 slice sweeps 1.61 -> 1.03 ms, ring_kernel 1.23).  With at most two
+// blocks nothing is left of the shorter chain where a phase's slices no longer fit on
+// the SMs, 16 warps each: ring_kernel has 64 registers (n = 24: P = 8, 3000 rings 0.56
+// here with 4 warps / 0.46 there; P = 24, 300 rings 0.35 / 0.29).  smem: a ring's shared
+// memory, cap: an SM's.
+inline int dense_warps(int P, int n, int rings, int sms, bool ref_order, size_t smem, size_t cap) {
     const int w = std::min(P, rings >= 2 * sms && n <= 256 ? 8 : 16);
     if (ref_order && P > 1) return w;
     const int phase = (P + 1) / 2;
     if (n <= 64 && rings > sms * (16 / phase)) return 0;
-    return rings > sms ? std::min(w, phase) : w;
+    if (rings <= sms) return w;
+    const int fit = std::max(1, (int)(cap / smem));
+    int best = 1;
+    double cost = 0.0;
+    for (int v = 1; v <= std::min(phase, 16); ++v) {
+        const double waves = std::ceil((double)rings / ((double)std::min(16 / v, fit) * sms));
+        const double c = waves * ((phase + v - 1) / v + 0.4);
+        if (v == 1 || c <= cost) {
+            best = v;
+            cost = c;
+        }
+    }
+    return best;
 }
 
 extern __shared__ __align__(16) unsigned char dense_sm[];

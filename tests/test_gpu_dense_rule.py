@@ -32,3 +32,14 @@ def test_checkerboard_matches_oracle(oracle, n, P, reads):
     finally:
         qa.set_update_order("reference")
         oracle.set_update_order("reference")
+
+
+@pytest.mark.parametrize("n,P,reads,warps", [
+    (84, 20, 371, 5),    # 3 rings an SM, 10 slices in two rounds: one wave (8 warps: two rounds as well, two waves)
+    (84, 20, 148, 16),   # no more rings than SMs
+    (400, 24, 450, 4),   # 4 rings an SM, as many as shared memory holds
+    (66, 12, 1200, 3)])
+def test_warps_by_waves_and_rounds(n, P, reads, warps):
+    from qlatanneal_b200 import _lib, autotune
+    eng = _lib.Engine.get(None)
+    assert autotune._ring_warps(eng, qa.DenseIsing(*dense_real(n, 1)), P, reads, True, False) == warps
