@@ -157,28 +157,39 @@ __device__ __noinline__ int hubo_sweep(const HubRows hr, uint32_t ordo, unsigned
             };
             uint32_t m = decide();
             if (m) {
-                auto chunk = [&](int j) {
-                    return hub_first(hr, __shfl_sync(FULL, hs.x, j), __shfl_sync(FULL, hs.y, j), lane);
+                uint32_t at, sizes, atn, sizesn;  // records and chunk sizes of spin j, of the next
+                auto chunk = [&](int j, uint32_t &x, uint32_t &y) {
+                    x = __shfl_sync(FULL, hs.x, j);
+                    y = __shfl_sync(FULL, hs.y, j);
+                    return hub_first(hr, x, y, lane);
                 };
                 int j = __ffs(m) - 1;
-                int4 rec = chunk(j);
+                int4 rec = chunk(j, at, sizes);
                 while (true) {
                     const uint32_t pend = j == 31 ? 0u : ~((2u << j) - 1u);
                     const int jj = __shfl_sync(FULL, i, j);
-                    const uint4 hj = hub_of(hs, j);
                     const int sj = __shfl_sync(FULL, sb, j) ? -1 : 1;  // the new spin
                     if (lane == 0) St[jj >> 5] ^= 1u << (jj & 31);
                     ++flips;
                     const int jn = (m & pend) ? __ffs(m & pend) - 1 : j;  // the likely next flip
-                    const int4 recn = chunk(jn);
+                    const int4 recn = chunk(jn, atn, sizesn);
                     __syncwarp();
                     hub_add(rec, gt, St, sj);
                     uint32_t touch = hubo_touch<ORD>(rec, inv, q);
-                    // (chunks in order: a target's terms stay in order)
-                    hub_chunks(hj, hr.size, hr.rec, lane, [&](const int4 &x) {
+                    auto further = [&](const int4 &x) {
                         hub_add(x, gt, St, sj);
                         touch |= hubo_touch<ORD>(x, inv, q);
-                    });
+                    };
+                    // (chunks in order: a target's terms stay in order; one further
+                    // chunk by itself: n = 226, P = 16, 50 rings, 81 sweeps 5.20 -> 4.88 ms)
+                    if (sizes >= 65536u) {
+                        hub_chunks(make_uint4(at, sizes, __shfl_sync(FULL, hs.z, j), __shfl_sync(FULL, hs.w, j)), hr.size,
+                                   hr.rec, lane, further);
+                    } else if (sizes >= 256u) {
+                        const int4 x = hub_first(hr, at + (sizes & 255u), sizes >> 8, lane);
+                        __syncwarp();
+                        further(x);
+                    }
                     touch = __reduce_or_sync(FULL, touch) & pend;
                     __syncwarp();
                     if (touch) {
@@ -186,9 +197,14 @@ __device__ __noinline__ int hubo_sweep(const HubRows hr, uint32_t ordo, unsigned
                         m = (m & ~touch) | (decide() & touch);
                     }
                     if (!(m & pend)) break;
-                    const int k = __ffs(m & pend) - 1;
-                    rec = k == jn ? recn : chunk(k);
-                    j = k;
+                    j = __ffs(m & pend) - 1;
+                    if (j == jn) {
+                        rec = recn;
+                        at = atn;
+                        sizes = sizesn;
+                    } else {
+                        rec = chunk(j, at, sizes);
+                    }
                 }
             }
             if (ORD) {
