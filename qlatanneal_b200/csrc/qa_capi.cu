@@ -1884,17 +1884,20 @@ static int sa_impl(qa_ctx *ctx, const qa_problem *const *problems, int n_problem
     bool real = kind == K_DENSE && !traces && !pm1 && sa_dense_smem_bytes<false>(n_max) <= (size_t)ctx->smem_optin &&
                 !std::getenv("QA_DISABLE_DENSE");
     for (int p = 0; p < n_problems && real; ++p) real = problems[p]->plain_j;
-    auto sa_kern = pm1 ? sa_dense_kernel<true> : sa_dense_kernel<false>;
+    auto sa_kern = pm1 ? sa_dense_kernel<true, false> : sa_dense_kernel<false, false>;
     const size_t sa_smem = pm1 ? sa_dense_smem_bytes<true>(n_max) : sa_dense_smem_bytes<false>(n_max);
     int sa_w = sa_warps(n_max);
     if (pm1 || real) {
         QA_TRY(opt_in_smem(ctx, (const void *)sa_kern, sa_smem));
         if (nr > ctx->sms) {
             int many = 0, one = 0;  // CTAs an SM
+            auto one_kern = pm1 ? sa_dense_kernel<true, true> : sa_dense_kernel<false, true>;
+            QA_TRY(opt_in_smem(ctx, (const void *)one_kern, sa_smem));
             QA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&many, sa_kern, 32 * sa_w, sa_smem));
-            QA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, sa_kern, 32, sa_smem));
+            QA_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&one, one_kern, 32, sa_smem));
             sa_w = sa_form(pm1, n_max, nr, (long long)many * ctx->sms, (long long)one * ctx->sms);
             real = real && sa_w > 0;
+            if (sa_w == 1) sa_kern = one_kern;
         }
     }
     QA_CK(cudaEventRecord(ctx->ev[0], ctx->stream));
