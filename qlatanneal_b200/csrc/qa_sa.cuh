@@ -43,10 +43,12 @@ static inline int sa_warps(int n) { return 1 + std::min(kSaWarps - 1, (n + 127) 
 // 2.72 -> 1.60.  +-1 from n = 400 on is bounded by shared memory either way (2%
 // slower with one warp).  Reads beyond that of small real models go to sa_kernel,
 // whose 64 registers hold 32 reads an SM against 12 here (n = 64, 4000 reads: one
-// warp 2.00, sa_kernel 1.62 ms; n = 128, 4700 reads: 3.93 and 4.42).
+// warp 2.00, sa_kernel 1.62 ms; n = 128, 4700 reads: 3.93 and 4.42), and the smallest
+// ones at once (n = 9, 829 reads 0.64 / 0.55; n = 17, 1445 reads 1.12 / 1.04; n = 19, 923
+// reads 0.119 / 0.125).
 static inline int sa_form(bool pm1, int n, long long nr, long long many, long long one) {
     if (nr <= (sa_warps(n) > 2 ? many : many / 2)) return sa_warps(n);
-    if (!pm1 && n < 96 && nr > one) return 0;
+    if (!pm1 && (n < 18 || (n < 96 && nr > one))) return 0;
     return one > many ? 1 : sa_warps(n);
 }
 

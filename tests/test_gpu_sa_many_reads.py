@@ -11,11 +11,12 @@ from test_gpu_parity_sa_sqa import oracle_model
 pytestmark = pytest.mark.gpu
 
 
-# either side of n = 96, of the 128 uniforms a warp draws and of 512 columns of a row; more
+# either side of n = 18, of n = 96, of the 128 uniforms a warp draws and of 512 columns of a row; more
 # reads than one warp a read holds (32 an SM at most) and fewer
 @pytest.mark.parametrize("kind,n,reads", [("pm1", 20, 5000), ("pm1", 129, 2500), ("real", 40, 1200), ("real", 40, 2600),
                                           ("real", 95, 2000), ("real", 96, 2000), ("real", 300, 900),
-                                          ("real", 514, 600), ("pm1", 1310, 700)])
+                                          ("real", 514, 600), ("pm1", 1310, 700), ("real", 17, 800),
+                                          ("real", 18, 800)])
 def test_many_reads_match_oracle(oracle, kind, n, reads):
     model = qa.DenseIsing(*(sk_dense(n, n, h_sigma=0.2) if kind == "pm1" else dense_real(n, n)))
     om = oracle_model(oracle, model)
