@@ -710,7 +710,8 @@ int plan_rings(qa_ctx *ctx, const qa_problem *const *probs, int np, int kind, in
         // P=32 10 rings 10.1 -> 8.8, n=64 P=32 one ring 6.5 -> 5.7) and more than
         // one block: a block of its own has no wavefront, and the further warps
         // cost (n=5 P=32 30 rings 19.2 -> 20.5 ms, n=32 0.97 to 1.04 of the speed
-        // by P, n=40 1.02 to 1.14)
+        // by P, n=40 1.02 to 1.14).  beta = P/2 throughout; where most spins flip
+        // n=512 1.09 to 1.31, but n<=256 P=32 0.95 to 0.99
         if (ref_order && ctx->tune.warps_per_ring <= 0 && P <= 32 &&
             (P <= 16 || (n_rings <= ctx->sms && n_max > 32) || 2 * pl->smem > (size_t)ctx->smem_optin))
             pl->W = P;
