@@ -9,7 +9,11 @@
 // the time.  Here the chains stay in shared memory for the whole run and a
 // barrier takes a launch's place; lane r of warp 0 holds slot r's energy in the
 // cascade.  n = 128, 24 rungs, 32 reads, 100 steps of 5 sweeps, swaps after each:
-// 9.8 -> 4.9 ms; n = 30 .. 400, 1 to 32 reads: 1.5 to 7 times faster.  What is left
+// 9.8 -> 4.9 ms; n = 30 .. 400, 1 to 32 reads: 1.5 to 7 times faster.  One SM for a
+// read's rungs costs less than the launches even where a launch per swap interval has
+// an SM for each rung and swaps are rare: 1 read, 32 rungs, swaps every 1000 steps,
+// n = 600 28 -> 25 ms, n = 8 3.7 -> 3.2 (1920 shapes, n = 8 .. 900, 2 to 32 rungs, 1 to
+// 200 reads, intervals of 1 to 1000 steps: none slower).  What is left
 // is the hottest chain of a read, whose blocks are chains of accepted flips
 // (limits on s g instead of the exponential after each: 5.7 -> 4.9 ms).
 #pragma once
